@@ -643,7 +643,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
 
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int n_tiles = C::GATED_SPLIT ? (p.N / 2 + C::BN / 2 - 1) / (C::BN / 2)
                                      : (p.N + C::BN - 1) / C::BN;
@@ -693,25 +693,28 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
 
   if (warp < 4) {
     if constexpr (C::REBALANCE_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-    if (warp == 0 && lane == 0) {
-      // ---------------- TMA producer ----------------
+    if (warp == 0) {
+      // ---------------- TMA producer (warp-uniform loop, one elected lane issues) ----------------
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       for (int t = sched_id; t < num_tiles && ok; t += sched_stride) {
         const TileCoord tc = decode_tile(sched, t);
         for (int kb = 0; kb < num_kb && ok; ++kb) {
-          ok = mbar_wait(&bars.empty[stage], phase ^ 1u, abort_p);
+          ok = mbar_wait_warp(&bars.empty[stage], phase ^ 1u, abort_p);
           if (!ok) break;
-          // the leader's barrier counts the bytes of both CTAs of a pair
-          if (rank == 0)
-            mbar_arrive_expect_tx(&bars.full[stage], C::STAGE_BYTES * (C::PAIR ? 2 : 1));
-          issue_stage<C>(map_a, map_b, p, tc, kb, rank, tiles + stage * C::STAGE_BYTES,
-                         &bars.full[stage]);
+          if (elect_one()) {
+            // the leader's barrier counts the bytes of both CTAs of a pair
+            if (rank == 0)
+              mbar_arrive_expect_tx(&bars.full[stage], C::STAGE_BYTES * (C::PAIR ? 2 : 1));
+            issue_stage<C>(map_a, map_b, p, tc, kb, rank, tiles + stage * C::STAGE_BYTES,
+                           &bars.full[stage]);
+          }
+          __syncwarp();
           if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
         }
       }
-    } else if (C::SCALED && warp == 1 && lane == 0) {
+    } else if (C::SCALED && warp == 1) {
       // ---------------- MMA issuer, scales applied by the tensor core ----------------
       // A scale word in tensor memory holds four e8m0 bytes per row, and an MMA picks one of
       // them by an index in its instruction descriptor.  A 128-block scale is the same for the
@@ -737,38 +740,44 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       uint32_t stage = 0, phase = 0, buf_phase = 0, group = 0;
       bool ok = true;
       for (int t = sched_id; t < num_tiles && ok; t += sched_stride) {
-        ok = mbar_wait(&bars.tempty[0], buf_phase ^ 1u, abort_p);  // the accumulator has been read out
+        ok = mbar_wait_warp(&bars.tempty[0], buf_phase ^ 1u, abort_p);  // the accumulator has been read out
         if (!ok) break;
         uint32_t accum = 0;
         for (int kb = 0; kb < num_kb && ok; ++kb) {
           const uint32_t j = static_cast<uint32_t>(kb) & 3u;
           if (j == 0) {  // next group of scale words: shared -> tensor memory
             const uint32_t g = group & 1u;
-            ok = mbar_wait(&bars.sffull[g], (group >> 1) & 1u, abort_p);
+            ok = mbar_wait_warp(&bars.sffull[g], (group >> 1) & 1u, abort_p);
             if (!ok) break;
             tc_fence_after();
             const uint32_t sf_lo = sf_lo0 + g * (kSfGroupBytes >> 4);
-            tmem_cp_32x128b_x4(sfa_t, desc(sf_lo, sf_hi));
-            tmem_cp_32x128b_x4(sfb_t, desc(sf_lo + (kSfaBytes >> 4), sf_hi));
-            tmem_cp_32x128b_x4(sfb_t + 4, desc(sf_lo + ((kSfaBytes + 512) >> 4), sf_hi));
-            mma_commit(&bars.sfempty[g]);  // the loader may refill once the copies are done
+            if (elect_one()) {
+              tmem_cp_32x128b_x4(sfa_t, desc(sf_lo, sf_hi));
+              tmem_cp_32x128b_x4(sfb_t, desc(sf_lo + (kSfaBytes >> 4), sf_hi));
+              tmem_cp_32x128b_x4(sfb_t + 4, desc(sf_lo + ((kSfaBytes + 512) >> 4), sf_hi));
+              mma_commit(&bars.sfempty[g]);  // the loader may refill once the copies are done
+            }
+            __syncwarp();
             ++group;
           }
-          ok = mbar_wait(&bars.full[stage], phase, abort_p);
+          ok = mbar_wait_warp(&bars.full[stage], phase, abort_p);
           if (!ok) break;
           tc_fence_after();
           const uint32_t a_lo = a_lo0 + stage * (C::STAGE_BYTES >> 4);
           const uint32_t b_lo = b_lo0 + stage * (C::STAGE_BYTES >> 4);
           const uint32_t idesc = idesc0 | (j << 4) | (j << 29);  // scale byte j for A and for B
-          mma_mxf8f6f4(tmem_base, desc(a_lo, sw_hi), desc(b_lo, sw_hi), idesc, sfa_t, sfb_t, accum);
-          mma_mxf8f6f4(tmem_base, desc(a_lo + 2, sw_hi), desc(b_lo + kBStep, sw_hi), idesc, sfa_t, sfb_t, 1u);
-          mma_mxf8f6f4(tmem_base, desc(a_lo + 4, sw_hi), desc(b_lo + 2 * kBStep, sw_hi), idesc, sfa_t, sfb_t, 1u);
-          mma_mxf8f6f4(tmem_base, desc(a_lo + 6, sw_hi), desc(b_lo + 3 * kBStep, sw_hi), idesc, sfa_t, sfb_t, 1u);
+          if (elect_one()) {
+            mma_mxf8f6f4(tmem_base, desc(a_lo, sw_hi), desc(b_lo, sw_hi), idesc, sfa_t, sfb_t, accum);
+            mma_mxf8f6f4(tmem_base, desc(a_lo + 2, sw_hi), desc(b_lo + kBStep, sw_hi), idesc, sfa_t, sfb_t, 1u);
+            mma_mxf8f6f4(tmem_base, desc(a_lo + 4, sw_hi), desc(b_lo + 2 * kBStep, sw_hi), idesc, sfa_t, sfb_t, 1u);
+            mma_mxf8f6f4(tmem_base, desc(a_lo + 6, sw_hi), desc(b_lo + 3 * kBStep, sw_hi), idesc, sfa_t, sfb_t, 1u);
+            mma_commit(&bars.empty[stage]);
+            if (kb + 1 == num_kb) mma_commit(&bars.tfull[0]);
+          }
+          __syncwarp();
           accum = 1;
-          mma_commit(&bars.empty[stage]);
           if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
         }
-        if (ok) mma_commit(&bars.tfull[0]);
         buf_phase ^= 1u;
       }
     } else if (C::SCALED && warp == 2) {
@@ -848,7 +857,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         }
       }
       if (__any_sync(0xffffffffu, bad) && lane == 0) atomicExch(&g_device_status, B200MOE_INVALID_ARG);
-    } else if (warp == 1 && lane == 0 && rank == 0) {
+    } else if (warp == 1 && rank == 0) {
       // ---------------- MMA issuer (the even CTA of a pair) ----------------
       const uint32_t idesc =
           make_idesc(p.ab_fmt, p.ab_fmt, 0u, C::B_MN_MAJOR ? 1u : 0u, C::TILE_M, C::BN);
@@ -869,16 +878,16 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
           // thread waits for; look at the operand stage first, so that wait is already behind
           // it when the buffer comes back.
           if constexpr (C::PROMOTE) {
-            ok = mbar_wait(&bars.full[stage], phase, abort_p);
+            ok = mbar_wait_warp(&bars.full[stage], phase, abort_p);
             if (!ok) break;
           }
-          ok = mbar_wait(&bars.tempty[buf], buf_phase ^ 1u, abort_p);
+          ok = mbar_wait_warp(&bars.tempty[buf], buf_phase ^ 1u, abort_p);
           if (!ok) break;
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + buf * C::BN;
           for (int kb = 0; kb < kb_per_phase && ok; ++kb) {
             if constexpr (!C::PROMOTE) {
-              ok = mbar_wait(&bars.full[stage], phase, abort_p);
+              ok = mbar_wait_warp(&bars.full[stage], phase, abort_p);
               if (!ok) break;
               tc_fence_after();
             }
@@ -887,27 +896,30 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
             // tensor pipe idles
             const uint32_t a_lo = a_lo0 + stage * (C::STAGE_BYTES >> 4);
             const uint32_t b_lo = b_lo0 + stage * (C::STAGE_BYTES >> 4);
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < C::BK / C::UMMA_K; ++kk) {
-              const uint64_t a_desc = (static_cast<uint64_t>(desc_hi) << 32) | (a_lo + kk * 2);
-              const uint64_t b_desc = (static_cast<uint64_t>(desc_hi) << 32) |
-                                      (b_lo + kk * (C::B_MN_MAJOR ? ((C::UMMA_K * kStageRowBytes) >> 4) : 2));
-              const uint32_t accum = (kb > 0 || kk > 0) ? 1u : 0u;
-              if constexpr (C::PAIR) {
-                if (C::KIND == KIND_F16) mma_f16_pair(d_tmem, a_desc, b_desc, idesc, accum);
-                else mma_f8_pair(d_tmem, a_desc, b_desc, idesc, accum);
-              } else {
-                if (C::KIND == KIND_F16) mma_f16(d_tmem, a_desc, b_desc, idesc, accum);
-                else mma_f8(d_tmem, a_desc, b_desc, idesc, accum);
+              for (int kk = 0; kk < C::BK / C::UMMA_K; ++kk) {
+                const uint64_t a_desc = (static_cast<uint64_t>(desc_hi) << 32) | (a_lo + kk * 2);
+                const uint64_t b_desc = (static_cast<uint64_t>(desc_hi) << 32) |
+                                        (b_lo + kk * (C::B_MN_MAJOR ? ((C::UMMA_K * kStageRowBytes) >> 4) : 2));
+                const uint32_t accum = (kb > 0 || kk > 0) ? 1u : 0u;
+                if constexpr (C::PAIR) {
+                  if (C::KIND == KIND_F16) mma_f16_pair(d_tmem, a_desc, b_desc, idesc, accum);
+                  else mma_f8_pair(d_tmem, a_desc, b_desc, idesc, accum);
+                } else {
+                  if (C::KIND == KIND_F16) mma_f16(d_tmem, a_desc, b_desc, idesc, accum);
+                  else mma_f8(d_tmem, a_desc, b_desc, idesc, accum);
+                }
+              }
+              if constexpr (C::PAIR) mma_commit_pair(&bars.empty[stage]);
+              else mma_commit(&bars.empty[stage]);
+              if (kb + 1 == kb_per_phase) {
+                if constexpr (C::PAIR) mma_commit_pair(&bars.tfull[buf]);
+                else mma_commit(&bars.tfull[buf]);
               }
             }
-            if constexpr (C::PAIR) mma_commit_pair(&bars.empty[stage]);
-            else mma_commit(&bars.empty[stage]);
+            __syncwarp();
             if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
-          }
-          if (ok) {
-            if constexpr (C::PAIR) mma_commit_pair(&bars.tfull[buf]);
-            else mma_commit(&bars.tfull[buf]);
           }
           if (++buf == C::ACC_BUFS) { buf = 0; buf_phase ^= 1u; }
         }

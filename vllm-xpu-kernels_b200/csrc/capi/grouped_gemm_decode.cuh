@@ -159,7 +159,7 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_tok,
 
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int n_out = GATED ? p.N / 2 : p.N;            // output features
   const int f_tiles = (n_out + kFeat - 1) / kFeat;
@@ -197,28 +197,31 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_tok,
   const int num_tiles = sched.tile_prefix[sched.num_experts];
   volatile int* abort_p = &abort_flag;
 
-  if (warp == 0 && lane == 0) {
-    // ---------------- TMA producer ----------------
+  if (warp == 0) {
+    // ---------------- TMA producer (warp-uniform loop, one elected lane issues) ----------------
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
       const DecodeTile tc = decode_tile(sched, t);
       for (int kb = 0; kb < num_kb && ok; ++kb) {
-        ok = mbar_wait(&bars.empty[stage], phase ^ 1u, abort_p);
+        ok = mbar_wait_warp(&bars.empty[stage], phase ^ 1u, abort_p);
         if (!ok) break;
         uint8_t* w_dst = tiles + stage * C::STAGE_BYTES;
         uint8_t* tok_dst = w_dst + C::W_TILES * kWBytes;
-        mbar_arrive_expect_tx(&bars.full[stage], C::STAGE_BYTES);
-        tma_load_3d(w_dst, &map_w, &bars.full[stage], tc.f_tile * kFeat, kb * kBK, tc.expert);
-        if (GATED)
-          tma_load_3d(w_dst + kWBytes, &map_w, &bars.full[stage], p.N / 2 + tc.f_tile * kFeat,
-                      kb * kBK, tc.expert);
-        tma_load_2d(tok_dst, &map_tok, &bars.full[stage], kb * kBK, tc.row_start);
+        if (elect_one()) {
+          mbar_arrive_expect_tx(&bars.full[stage], C::STAGE_BYTES);
+          tma_load_3d(w_dst, &map_w, &bars.full[stage], tc.f_tile * kFeat, kb * kBK, tc.expert);
+          if (GATED)
+            tma_load_3d(w_dst + kWBytes, &map_w, &bars.full[stage], p.N / 2 + tc.f_tile * kFeat,
+                        kb * kBK, tc.expert);
+          tma_load_2d(tok_dst, &map_tok, &bars.full[stage], kb * kBK, tc.row_start);
+        }
+        __syncwarp();
         if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
       }
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     // A = weights, MN-major (features contiguous); B = tokens, K-major; e4m3 x e4m3 -> fp32
     const uint32_t idesc = make_idesc(0u, 0u, 1u, 0u, kFeat, kNTok);
@@ -232,9 +235,9 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_tok,
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
       for (int kb = 0; kb < num_kb && ok; ++kb) {
-        ok = mbar_wait(&bars.tempty[buf], buf_phase ^ 1u, abort_p);
+        ok = mbar_wait_warp(&bars.tempty[buf], buf_phase ^ 1u, abort_p);
         if (!ok) break;
-        ok = mbar_wait(&bars.full[stage], phase, abort_p);
+        ok = mbar_wait_warp(&bars.full[stage], phase, abort_p);
         if (!ok) break;
         tc_fence_after();
         // descriptors: constant high word, low words = base + stage * constant (+ an
@@ -243,19 +246,22 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_tok,
         const uint32_t w_lo = w_lo0 + stage * (C::STAGE_BYTES >> 4);
         const uint32_t tok_lo = tok_lo0 + stage * (C::STAGE_BYTES >> 4);
         const uint32_t d_tmem = tmem_base + buf * C::ACC_COLS;
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          const uint64_t b_desc = (static_cast<uint64_t>(desc_hi) << 32) | (tok_lo + kk * 2);
-          const uint64_t a_gate = (static_cast<uint64_t>(desc_hi) << 32) | (w_lo + kk * ((32 * 128) >> 4));
-          mma_f8(d_tmem, a_gate, b_desc, idesc, kk > 0 ? 1u : 0u);
-          if (GATED) {
-            const uint64_t a_up = (static_cast<uint64_t>(desc_hi) << 32) |
-                                  (w_lo + (kWBytes >> 4) + kk * ((32 * 128) >> 4));
-            mma_f8(d_tmem + kNTok, a_up, b_desc, idesc, kk > 0 ? 1u : 0u);
+          for (int kk = 0; kk < 4; ++kk) {
+            const uint64_t b_desc = (static_cast<uint64_t>(desc_hi) << 32) | (tok_lo + kk * 2);
+            const uint64_t a_gate = (static_cast<uint64_t>(desc_hi) << 32) | (w_lo + kk * ((32 * 128) >> 4));
+            mma_f8(d_tmem, a_gate, b_desc, idesc, kk > 0 ? 1u : 0u);
+            if (GATED) {
+              const uint64_t a_up = (static_cast<uint64_t>(desc_hi) << 32) |
+                                    (w_lo + (kWBytes >> 4) + kk * ((32 * 128) >> 4));
+              mma_f8(d_tmem + kNTok, a_up, b_desc, idesc, kk > 0 ? 1u : 0u);
+            }
           }
+          mma_commit(&bars.empty[stage]);
+          mma_commit(&bars.tfull[buf]);
         }
-        mma_commit(&bars.empty[stage]);
-        mma_commit(&bars.tfull[buf]);
+        __syncwarp();
         if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
         if (++buf == C::ACC_BUFS) { buf = 0; buf_phase ^= 1u; }
       }

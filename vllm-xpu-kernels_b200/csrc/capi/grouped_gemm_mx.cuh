@@ -162,7 +162,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
                                                ~static_cast<uintptr_t>(1023));
   uint8_t* sfa_smem = tiles + C::STAGES * C::STAGE_BYTES;
   uint8_t* sfb_smem = sfa_smem + C::STAGES * kMxSfaBytes;
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int n_tiles = (p.N + C::BN - 1) / C::BN;
   const int num_kb = (p.K + kMxBK - 1) / kMxBK;
@@ -199,8 +199,8 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
   const int sched_id = blockIdx.x, sched_stride = gridDim.x;
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------- TMA producer ----------------
+    {
+      // ---------------- TMA producer (warp-uniform loop, one elected lane issues) ----------------
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -210,23 +210,26 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
         const uint8_t* sfb_tile =
             p.b_sf + (static_cast<int64_t>(tc.expert) * num_kb * p.b_atoms + n0 / 128) * kMxAtomBytes;
         for (int kb = 0; kb < num_kb && ok; ++kb) {
-          ok = mbar_wait_spin(&bars.empty[stage], phase ^ 1u, abort_p);
+          ok = mbar_wait_warp(&bars.empty[stage], phase ^ 1u, abort_p);
           if (!ok) break;
           const bool tail = tail_skip && kb == num_kb - 1;
           uint8_t* a_dst = tiles + stage * C::STAGE_BYTES;
-          mbar_arrive_expect_tx(&bars.full[stage], C::STAGE_TX_BYTES + C::SFB_BYTES);
-          tma_load_2d(a_dst, &map_a, &bars.full[stage], tail ? p.K - kMxBK : kb * kMxBK, tc.row_start);
-          if (tail) tma_load_3d(a_dst + C::A_BYTES, &map_b_tail, &bars.full[stage], 0, n0, tc.expert);
-          else tma_load_3d(a_dst + C::A_BYTES, &map_b, &bars.full[stage], kb * kMxBK, n0, tc.expert);
-          bulk_load(sfb_smem + stage * C::SFB_BYTES,
-                    sfb_tile + static_cast<int64_t>(kb) * p.b_atoms * kMxAtomBytes, C::SFB_BYTES,
-                    &bars.full[stage]);
+          if (elect_one()) {
+            mbar_arrive_expect_tx(&bars.full[stage], C::STAGE_TX_BYTES + C::SFB_BYTES);
+            tma_load_2d(a_dst, &map_a, &bars.full[stage], tail ? p.K - kMxBK : kb * kMxBK, tc.row_start);
+            if (tail) tma_load_3d(a_dst + C::A_BYTES, &map_b_tail, &bars.full[stage], 0, n0, tc.expert);
+            else tma_load_3d(a_dst + C::A_BYTES, &map_b, &bars.full[stage], kb * kMxBK, n0, tc.expert);
+            bulk_load(sfb_smem + stage * C::SFB_BYTES,
+                      sfb_tile + static_cast<int64_t>(kb) * p.b_atoms * kMxAtomBytes, C::SFB_BYTES,
+                      &bars.full[stage]);
+          }
+          __syncwarp();
           if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
       // ---------------- MMA issuer ----------------
       // One thread feeds the tensor pipe, and an MMA of this shape takes about 100 cycles:
       // the scalar instructions between two tcgen05.mma decide whether the pipe stays busy.
@@ -262,42 +265,45 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
             // a tile that starts inside a 128-row piece of the scales (192-column tiles: every
             // odd one starts at row 64) reads its scale columns from that offset on
             sfb_t = tmem_base + kMxSfbCol + ((n_tile * C::BN) % 128) / 32;
-            ok = mbar_wait(&bars.tempty[buf], buf_phase ^ 1u, abort_p);
+            ok = mbar_wait_warp(&bars.tempty[buf], buf_phase ^ 1u, abort_p);
             if (!ok) break;
             d_tmem = tmem_base + buf * C::ACC_STRIDE;
             accum = 0;
           }
-          ok = mbar_wait_spin(&bars.full[s], phase, abort_p);
+          ok = mbar_wait_warp(&bars.full[s], phase, abort_p);
           if (!ok) break;
           tc_fence_after();
-          tmem_cp_32x128b_x4(sfa_t, desc(sfa_lo0 + s * (kMxSfaBytes >> 4), sf_hi));
-#pragma unroll
-          for (int a = 0; a < C::B_ATOMS; ++a)
-            tmem_cp_32x128b_x4(tmem_base + kMxSfbCol + 4 * a,
-                               desc(sfb_lo0 + (s * C::SFB_BYTES + a * kMxAtomBytes) / 16, sf_hi));
           const uint32_t a_lo = a_lo0 + s * (C::STAGE_BYTES >> 4);
           const uint32_t b_lo = b_lo0 + s * (C::STAGE_BYTES >> 4);
-          if (tail_skip && kb == num_kb - 1) {
-            // K % 128 == 64 (rows of packed 4-bit weights have a 32-byte pitch, so K is a multiple
-            // of 64): the stage was loaded at K-128 and its first two sub-blocks were issued with
-            // the stage before
-            mma_mxf8f6f4(d_tmem, desc(a_lo + 4, sw_hi), desc(b_lo + 4, sw_hi),
-                         make_idesc_mx(0u, 5u, 0u, BM, C::BN, 2, 2), sfa_t, sfb_t, accum);
-            mma_mxf8f6f4(d_tmem, desc(a_lo + 6, sw_hi), desc(b_lo + 6, sw_hi),
-                         make_idesc_mx(0u, 5u, 0u, BM, C::BN, 3, 3), sfa_t, sfb_t, 1u);
-            accum = 1;
-          } else {
-            mma_mxf8f6f4(d_tmem, desc(a_lo, sw_hi), desc(b_lo, sw_hi),
-                         make_idesc_mx(0u, 5u, 0u, BM, C::BN, 0, 0), sfa_t, sfb_t, accum);
-            accum = 1;
+          const bool last = kb == num_kb - 1;
+          if (elect_one()) {
+            tmem_cp_32x128b_x4(sfa_t, desc(sfa_lo0 + s * (kMxSfaBytes >> 4), sf_hi));
 #pragma unroll
-            for (int kk = 1; kk < 4; ++kk)
-              mma_mxf8f6f4(d_tmem, desc(a_lo + kk * 2, sw_hi), desc(b_lo + kk * 2, sw_hi),
-                           make_idesc_mx(0u, 5u, 0u, BM, C::BN, kk, kk), sfa_t, sfb_t, 1u);
+            for (int a = 0; a < C::B_ATOMS; ++a)
+              tmem_cp_32x128b_x4(tmem_base + kMxSfbCol + 4 * a,
+                                 desc(sfb_lo0 + (s * C::SFB_BYTES + a * kMxAtomBytes) / 16, sf_hi));
+            if (tail_skip && last) {
+              // K % 128 == 64 (rows of packed 4-bit weights have a 32-byte pitch, so K is a
+              // multiple of 64): the stage was loaded at K-128 and its first two sub-blocks were
+              // issued with the stage before
+              mma_mxf8f6f4(d_tmem, desc(a_lo + 4, sw_hi), desc(b_lo + 4, sw_hi),
+                           make_idesc_mx(0u, 5u, 0u, BM, C::BN, 2, 2), sfa_t, sfb_t, accum);
+              mma_mxf8f6f4(d_tmem, desc(a_lo + 6, sw_hi), desc(b_lo + 6, sw_hi),
+                           make_idesc_mx(0u, 5u, 0u, BM, C::BN, 3, 3), sfa_t, sfb_t, 1u);
+            } else {
+              mma_mxf8f6f4(d_tmem, desc(a_lo, sw_hi), desc(b_lo, sw_hi),
+                           make_idesc_mx(0u, 5u, 0u, BM, C::BN, 0, 0), sfa_t, sfb_t, accum);
+#pragma unroll
+              for (int kk = 1; kk < 4; ++kk)
+                mma_mxf8f6f4(d_tmem, desc(a_lo + kk * 2, sw_hi), desc(b_lo + kk * 2, sw_hi),
+                             make_idesc_mx(0u, 5u, 0u, BM, C::BN, kk, kk), sfa_t, sfb_t, 1u);
+            }
+            mma_commit(&bars.empty[s]);
+            if (last) mma_commit(&bars.tfull[buf]);
           }
-          mma_commit(&bars.empty[s]);
+          __syncwarp();
+          accum = 1;
           if (++kb == num_kb) {
-            mma_commit(&bars.tfull[buf]);
             kb = 0;
             if (++buf == 2) { buf = 0; buf_phase ^= 1u; }
             t += sched_stride;

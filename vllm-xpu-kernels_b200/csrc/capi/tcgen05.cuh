@@ -85,6 +85,31 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   }
 }
 
+// The same wait by a whole converged warp; every lane gets the same answer.  The loops that
+// issue TMA loads and MMAs run warp-uniformly and elect one lane for the asynchronous
+// instruction alone: a loop inside `if (lane == 0)` makes the compiler treat barrier addresses,
+// descriptors and coordinates as per-thread values, and each of those instructions, which take
+// uniform registers, then costs a move per operand.  Measured per pipeline step (cycles): wait +
+// expect_tx + one TMA load 490 -> 264, with four loads 786 -> 388; wait + four MMAs + commit
+// 482 -> 207 (an MMA of 128 x 128 x 32 bytes of K itself takes 64, one of 128 x 256 takes 128).
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity,
+                                               volatile int* abort_flag) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const long long t0 = clock64();
+  while (true) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if (__any_sync(0xffffffffu, *abort_flag != 0 || clock64() - t0 > kWaitBudgetCycles)) {
+      *abort_flag = 1;
+      return false;
+    }
+  }
+}
+
+// Warp index as a value the compiler knows to be the same in all lanes.
+__device__ __forceinline__ int warp_index() {
+  return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
+}
+
 // Same contract for a wait that is off every critical path (many thousand cycles long, and a
 // microsecond late costs nothing): sleeps between polls, so the warp takes no issue slots
 // from the warps that share its scheduler.
