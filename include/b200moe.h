@@ -121,7 +121,8 @@ int b200moe_topk_softplus_sqrt(const void* logits, int in_dtype, int T, int E, i
 /* ---- permutation ------------------------------------------------------ */
 
 /* moe_align_block_size (csrc/moe/torch_bindings.cpp:14-20,
- * csrc/moe/moe_align_sum_kernels.cpp:1034-1181).  topk_ids: `numel` entries of
+ * csrc/moe/moe_align_sum_kernels.cpp:1034-1181).  The workspace is not read or
+ * written any more (the counts stay in shared memory) and may be NULL.  topk_ids: `numel` entries of
  * `ids_dtype`; expert_map i32 [num_experts] or NULL.  sorted_token_ids has
  * `sorted_capacity` entries, expert_ids `blocks_capacity`.  Order inside an
  * expert is ascending flat index (stable), so the result is reproducible. */
@@ -140,15 +141,9 @@ int b200moe_moe_align_block_size(const void* topk_ids, int ids_dtype,
  * path, a C host with no allocator to lend a workspace from.  It has no
  * counterpart in vllm-xpu-kernels (whose operator allocates its scratch with
  * torch).  Same arguments and results as b200moe_moe_align_block_size minus the
- * workspace: the scratch is a 256 KiB array built into the library (every GPU
- * that loads the library carries it until the process ends).
+ * workspace (the grouping keeps its counts in shared memory).
  *   Limit: ceil(numel / 2048) * num_experts <= 65536; larger problems get
  *   B200MOE_WORKSPACE_TOO_SMALL and a message in b200moe_last_error().
- *   The first call on each device looks the array's device address up once, with
- *   that device current; make that first call before any stream capture.
- *   All calls on a device share the array: two calls whose kernels can overlap
- *   on the GPU (different streams) race; calls on one stream are safe, and
- *   nothing needs clearing between them.
  * Calls no cudaMalloc / cudaFree or allocating library routine. */
 int b200moe_moe_align_block_size_static(const void* topk_ids, int ids_dtype,
                                         int64_t numel, int num_experts,
@@ -452,6 +447,52 @@ int b200moe_selftest_wait_timeout(long long budget_cycles, void* stream);
 /* Reads (and clears) the sticky device status word that bounded waits inside
  * the tensor-core kernels set when they give up; 0 = none.  Synchronises. */
 int b200moe_device_status(void* stream, int* status_host);
+
+/* ---- the whole layer --------------------------------------------------------------
+ * XpuFusedMoe.apply (vllm_xpu_kernels/fused_moe_interface.py:333-492) as one call:
+ * permute (with the activation quantisation, when x is 16-bit and the recipe takes
+ * quantised rows) -> grouped GEMM w13 with the gated activation in its epilogue ->
+ * grouped GEMM w2 -> weighted combine.  Launches kernels only; all scratch is the
+ * caller's workspace, which may be reused as soon as the stream has passed the call. */
+typedef struct b200moe_layer {
+  int recipe;        /* BF16, FP8_BLOCK or MXFP4 (scales from b200moe_mx_prepare_weight_scales) */
+  int epilogue;      /* of the first GEMM: SILU_MUL or SWIGLU_OAI                  */
+  int b_layout;      /* BF16 recipe: B200MOE_B_LAYOUT_*                            */
+  int gated_act;     /* SILU_MUL: B200MOE_ACT_*                                    */
+  float act_param0, act_param1, clamp_limit, alpha, limit;
+  int scales_pow2;   /* FP8_BLOCK: all weight scales are powers of two             */
+  int H, I, E;       /* hidden, intermediate, local experts                        */
+  const void *w13, *w13_scale, *w13_bias;
+  const void *w2, *w2_scale, *w2_bias;
+  int w13_bias_dtype, w2_bias_dtype;
+} b200moe_layer;
+
+#define B200MOE_LAYER_PERMUTE 1
+#define B200MOE_LAYER_GEMM1 2
+#define B200MOE_LAYER_GEMM2 4
+#define B200MOE_LAYER_COMBINE 8
+#define B200MOE_LAYER_ALL 15
+
+typedef struct b200moe_layer_call {
+  int stages;        /* B200MOE_LAYER_* bits; a pass may be split over several calls
+                        with the same workspace, in order                          */
+  const void* x;     /* [T,H] bf16 / f16, or e4m3 with x_scale                     */
+  int x_dtype;
+  const void* x_scale; /* FP8_BLOCK: f32 [T,H/128]; MXFP4: e8m0 [T,16*ceil(H/512)]  */
+  const float* topk_weights; /* [T,k]                                              */
+  const void* topk_ids;      /* [T,k] of ids_dtype, global expert ids              */
+  int ids_dtype;
+  const int32_t* expert_map; /* global id -> local id or -1; NULL: ids are local   */
+  int T, k, total_experts;
+  void* out;         /* [T,H] bf16 / f16                                           */
+  int out_dtype;
+  const void* shared;          /* optional [T,H] rows added with weight 1          */
+  const int32_t* valid_tokens; /* optional, see b200moe_moe_gather_bounded         */
+} b200moe_layer_call;
+
+size_t b200moe_layer_workspace_bytes(const b200moe_layer* layer, const b200moe_layer_call* call);
+int b200moe_layer_forward(const b200moe_layer* layer, const b200moe_layer_call* call,
+                          void* workspace, size_t workspace_bytes, void* stream);
 
 /* ---- expert-parallel exchange over peer-mapped memory -------------------------
  * vllm-xpu-kernels has no exchange step (its expert-parallel mode masks

@@ -5,6 +5,7 @@
 Produces, next to the Python package:
   vllm_xpu_kernels/libb200moe.so     CUDA kernels + C ABI (nvcc, sm_100a only)
   vllm_xpu_kernels/_b200_torch_ops.so  torch operator registry (g++), links the above
+  vllm_xpu_kernels/_b200_layer.so    CPython entry of the whole-layer call (g++), links the above
 
 Objects are cached under build/ by source hash, so a second run only relinks
 what changed.  nvcc cross-compiles: no GPU is needed to build.
@@ -18,7 +19,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CAPI = os.path.join(HERE, "csrc", "capi")
-TORCH_SRC = os.path.join(HERE, "csrc", "torch", "bindings.cpp")
+TORCH_DIR = os.path.join(HERE, "csrc", "torch")
 PKG = os.path.join(HERE, "vllm_xpu_kernels")
 BUILD = os.path.join(HERE, "build")
 INCLUDE = os.path.join(ROOT, "include")
@@ -70,32 +71,43 @@ def build_capi(force=False):
     return lib
 
 
-def build_torch_ops(force=False):
+def _build_torch_lib(source, name, extra_libs, force):
+    import sysconfig
+
     import torch
     from torch.utils import cpp_extension as ce
-    out = os.path.join(PKG, "_b200_torch_ops.so")
-    stamp = os.path.join(BUILD, "torch_ops.stamp")
-    want = _hash([TORCH_SRC, os.path.join(INCLUDE, "b200moe.h")], torch.__version__)
+    src = os.path.join(TORCH_DIR, source)
+    out = os.path.join(PKG, name + ".so")
+    stamp = os.path.join(BUILD, name + ".stamp")
+    want = _hash([src, os.path.join(INCLUDE, "b200moe.h")], torch.__version__)
     if not force and os.path.exists(out) and os.path.exists(stamp) and open(stamp).read() == want:
         return out
     inc = []
-    for p in ce.include_paths() + ["/usr/local/cuda/include", INCLUDE]:
+    for p in ce.include_paths() + ["/usr/local/cuda/include", INCLUDE, sysconfig.get_paths()["include"]]:
         inc += ["-I", p]
     tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-D_GLIBCXX_USE_CXX11_ABI=%d" % abi,
-           "-DTORCH_EXTENSION_NAME=_b200_torch_ops"] + inc + [TORCH_SRC, "-o", out + ".tmp",
+           "-DTORCH_EXTENSION_NAME=" + name] + inc + [src, "-o", out + ".tmp",
            "-L", tlib, "-L", PKG, "-L", "/usr/local/cuda/lib64",
-           "-lc10", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-ltorch_cuda", "-lb200moe", "-lcudart",
-           "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + tlib]
+           "-lc10", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-ltorch_cuda"] + extra_libs + [
+           "-lb200moe", "-lcudart", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + tlib]
     _run(cmd)
     os.replace(out + ".tmp", out)
     open(stamp, "w").write(want)
     return out
 
 
+def build_torch_ops(force=False):
+    return _build_torch_lib("bindings.cpp", "_b200_torch_ops", [], force)
+
+
+def build_layer(force=False):
+    return _build_torch_lib("layer.cpp", "_b200_layer", ["-ltorch_python"], force)
+
+
 def build_all(force=False):
-    return build_capi(force), build_torch_ops(force)
+    return build_capi(force), build_torch_ops(force), build_layer(force)
 
 
 if __name__ == "__main__":

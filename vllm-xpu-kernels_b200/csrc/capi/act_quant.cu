@@ -7,6 +7,7 @@
 // over the data.  Math is plain IEEE fp32 (no fast-math) so the scale formulas
 // give the same bits as a straightforward fp32 evaluation.
 #include "common.cuh"
+#include "quant_math.cuh"
 
 namespace b200moe {
 namespace {
@@ -153,17 +154,6 @@ __global__ void __launch_bounds__(256) relu2_kernel(T* __restrict__ out, const T
 }
 
 // ---- group quantisation ---------------------------------------------------
-
-__device__ __forceinline__ float round_up_pow2(float s) {
-  return exp2f(ceilf(log2f(fmaxf(fabsf(s), 1e-10f))));
-}
-
-template <int LANES>
-__device__ __forceinline__ float seg_max(float v) {
-#pragma unroll
-  for (int off = 1; off < LANES; off <<= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
-  return v;
-}
 
 __device__ __forceinline__ float seg_max_dyn(float v, int lanes) {
   for (int off = 1; off < lanes; off <<= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));

@@ -18,6 +18,8 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(
     const int32_t* __restrict__ num_valid, int k, int H) {
   constexpr int V = 16 / sizeof(T);
   const int64_t t = blockIdx.x;
+  pdl_wait();
+  pdl_trigger();
   if (num_valid && t >= *num_valid) return;  // rows of a worst-case buffer nobody will read
   __shared__ int rows[kMaxTopK];
   __shared__ float w[kMaxTopK];
@@ -53,6 +55,8 @@ __global__ void __launch_bounds__(256) moe_sum_kernel(
     int ids_dtype, const int32_t* __restrict__ expert_map) {
   const int64_t t = blockIdx.x;
   __shared__ int keep[kMaxTopK];
+  pdl_wait();
+  pdl_trigger();
   for (int j = threadIdx.x; j < k; j += blockDim.x) {
     int kp = 1;
     if (ids) {
@@ -93,10 +97,10 @@ static int gather_impl(void* out, const void* y, int dtype, const float* weights
     constexpr int V = 16 / sizeof(scalar_t);
     int threads = (H / V + 31) / 32 * 32;
     threads = threads > 256 ? 256 : threads;
-    moe_gather_kernel<scalar_t><<<T, threads, 0, as_stream(stream)>>>(
-        reinterpret_cast<scalar_t*>(out), reinterpret_cast<const scalar_t*>(y), weights, row_map,
-        reinterpret_cast<const scalar_t*>(addend), num_valid, k, H);
-    return launch_status("moe_gather_kernel");
+    return launch_pdl("moe_gather_kernel", moe_gather_kernel<scalar_t>, dim3(T), dim3(threads), 0,
+                      as_stream(stream), 1, reinterpret_cast<scalar_t*>(out),
+                      reinterpret_cast<const scalar_t*>(y), weights, row_map,
+                      reinterpret_cast<const scalar_t*>(addend), num_valid, k, H);
   });
 }
 
@@ -131,15 +135,10 @@ extern "C" int b200moe_moe_sum(const void* in, void* out, int dtype, int T, int 
     cudaStream_t st = as_stream(stream);
     const scalar_t* i = reinterpret_cast<const scalar_t*>(in);
     scalar_t* o = reinterpret_cast<scalar_t*>(out);
-    if (H % VMAX == 0) {
-      int threads = (H / VMAX + 31) / 32 * 32;
-      threads = threads > 256 ? 256 : threads;
-      moe_sum_kernel<scalar_t, VMAX><<<T, threads, 0, st>>>(o, i, k, H, topk_ids, ids_dtype, expert_map);
-    } else {
-      int threads = (H + 31) / 32 * 32;
-      threads = threads > 256 ? 256 : threads;
-      moe_sum_kernel<scalar_t, 1><<<T, threads, 0, st>>>(o, i, k, H, topk_ids, ids_dtype, expert_map);
-    }
-    return launch_status("moe_sum_kernel");
+    const bool vec = H % VMAX == 0;
+    int threads = ((vec ? H / VMAX : H) + 31) / 32 * 32;
+    threads = threads > 256 ? 256 : threads;
+    return launch_pdl("moe_sum_kernel", vec ? moe_sum_kernel<scalar_t, VMAX> : moe_sum_kernel<scalar_t, 1>, dim3(T),
+                      dim3(threads), 0, st, 1, o, i, k, H, topk_ids, ids_dtype, expert_map);
   });
 }

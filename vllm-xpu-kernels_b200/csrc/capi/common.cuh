@@ -60,6 +60,47 @@ int ensure_dynamic_smem(Kernel kernel, size_t bytes, const char* what) {
   return B200MOE_OK;
 }
 
+// ---- programmatic dependent launch ---------------------------------------------------
+// A kernel launched this way may become resident while the kernel before it in the stream is
+// still running, so its launch latency and its prologue (barriers, tensor memory, descriptor
+// prefetch) overlap the predecessor's tail; what it reads or writes waits in pdl_wait(), which
+// returns when every earlier kernel of the stream is complete and its writes are visible.
+// Every kernel launched this way calls pdl_wait() before pdl_trigger() in all its threads, so
+// at most two neighbouring kernels of a stream overlap, and a kernel that has not passed
+// pdl_wait() touches no memory another kernel writes.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... KArgs, typename... Args>
+int launch_pdl(const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+               cudaStream_t st, unsigned cluster, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cluster > 1) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
+  count_launch();
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    set_last_error(what, e);
+    return B200MOE_CUDA_ERROR;
+  }
+  return B200MOE_OK;
+}
+
 template <typename T> struct Elem;
 template <> struct Elem<float> {
   static __device__ __forceinline__ float to_f32(float v) { return v; }

@@ -670,6 +670,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     prefetch_tensormap(&map_a);
     prefetch_tensormap(&map_b);
   }
+  pdl_wait();   // everything below reads what earlier kernels wrote
+  pdl_trigger();
   build_schedule(sched, p.rows_per_expert, p.E, p.R, n_tiles, C::TILE_M);
   if (warp == 1) {
     if constexpr (C::PAIR) {
@@ -1218,29 +1220,9 @@ int launch_config(const b200moe_gemm_args& a, const void* B, int b_dtype, cudaSt
     if (c >= 2 && c < grid) grid = c;
   }
   if (grid < 1) grid = 1;
-  if (C::PAIR) {
-    grid = grid < 2 ? 2 : grid & ~1ll;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(grid));
-    cfg.blockDim = dim3(C::THREADS);
-    cfg.dynamicSmemBytes = C::SMEM_BYTES;
-    cfg.stream = st;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, grouped_gemm_kernel<C>, map_a, map_b, p);
-    if (e != cudaSuccess) {
-      set_last_error("grouped_gemm_kernel (cluster launch)", e);
-      return B200MOE_CUDA_ERROR;
-    }
-    return launch_status("grouped_gemm_kernel");
-  }
-  grouped_gemm_kernel<C><<<static_cast<int>(grid), C::THREADS, C::SMEM_BYTES, st>>>(map_a, map_b, p);
-  return launch_status("grouped_gemm_kernel");
+  if (C::PAIR) grid = grid < 2 ? 2 : grid & ~1ll;
+  return launch_pdl("grouped_gemm_kernel", grouped_gemm_kernel<C>, dim3(static_cast<unsigned>(grid)),
+                    dim3(C::THREADS), C::SMEM_BYTES, st, C::PAIR ? 2 : 1, map_a, map_b, p);
 }
 
 // ---- CUDA-core evaluation of the same contract (checking aid) --------------------------

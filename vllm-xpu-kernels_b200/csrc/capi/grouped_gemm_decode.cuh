@@ -185,6 +185,8 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_tok,
     prefetch_tensormap(&map_tok);
     prefetch_tensormap(&map_w);
   }
+  pdl_wait();
+  pdl_trigger();
   build_decode_schedule(sched, p.rows_per_expert, p.E, p.R, f_tiles);
   if (warp == 1) {
     tmem_alloc(&tmem_base_slot, C::TMEM_COLS);
@@ -447,8 +449,8 @@ int launch_decode(const b200moe_gemm_args& a, cudaStream_t st) {
       decode_gemm_kernel<GATED>, C::SMEM_BYTES + kMaxDecodeKBlocks * (kNTok + 2) * sizeof(float),
       "cudaFuncSetAttribute");
   if (arc != B200MOE_OK) return arc;
-  decode_gemm_kernel<GATED><<<kNumSMs, C::THREADS, smem, st>>>(map_tok, map_w, p);
-  return launch_status("decode_gemm_kernel");
+  return launch_pdl("decode_gemm_kernel", decode_gemm_kernel<GATED>, dim3(kNumSMs), dim3(C::THREADS), smem, st, 1,
+                    map_tok, map_w, p);
 }
 
 // Entry used by b200moe_grouped_gemm when the caller asks for the decode form

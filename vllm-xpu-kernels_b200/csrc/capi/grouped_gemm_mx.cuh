@@ -185,6 +185,8 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
     prefetch_tensormap(&map_b);
     prefetch_tensormap(&map_b_tail);
   }
+  pdl_wait();
+  pdl_trigger();
   build_schedule(sched, p.rows_per_expert, p.E, p.R, n_tiles, BM);
   if (warp == 1) {
     tmem_alloc(&tmem_base_slot, C::TMEM_COLS);
@@ -474,9 +476,8 @@ int launch_mx(const b200moe_mx_gemm_args& a, cudaStream_t st) {
   int64_t grid = ((a.R + BM - 1) / BM + a.E) * n_tiles;
   if (grid > kNumSMs) grid = kNumSMs;
   if (grid < 1) grid = 1;
-  grouped_gemm_mx_kernel<C><<<static_cast<int>(grid), C::THREADS, C::SMEM_BYTES, st>>>(
-      map_a, map_b, map_b_tail, p);
-  return launch_status("grouped_gemm_mx_kernel");
+  return launch_pdl("grouped_gemm_mx_kernel", grouped_gemm_mx_kernel<C>, dim3(static_cast<unsigned>(grid)),
+                    dim3(C::THREADS), C::SMEM_BYTES, st, 1, map_a, map_b, map_b_tail, p);
 }
 
 // Weight scales [E, N, K/32] (e8m0 bytes) -> [E, ceil(K/128), ceil(N/128)+1, 512]: per

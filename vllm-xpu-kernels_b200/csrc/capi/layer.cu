@@ -1,0 +1,188 @@
+// The whole fused-MoE layer as one host call: permute (+ activation quantisation) -> grouped
+// GEMM w13 (gated activation in its epilogue) -> grouped GEMM w2 -> weighted combine.
+//
+// With few tokens the layer is a chain of short kernels and what the host does between two
+// launches is on the critical path: one call from the framework's side instead of ten, one
+// scratch buffer instead of seven, and five launches (four when the grouping is done inside
+// the row kernel) that each overlap their prologue with the kernel before them.
+#include <stdlib.h>
+
+#include "common.cuh"
+#include "layer.cuh"
+
+namespace b200moe {
+namespace {
+
+constexpr size_t kAlign = 256;
+
+struct Workspace {
+  size_t rows, row_scales, act, act_scales, out, counts, row_map, total;
+};
+
+size_t mx_pitch(int64_t width) { return static_cast<size_t>((width + 511) / 512) * 16; }
+
+Workspace carve(const b200moe_layer* l, const b200moe_layer_call* c) {
+  const size_t R = static_cast<size_t>(c->T) * c->k, H = l->H, I = l->I;
+  Workspace w{};
+  size_t at = 0;
+  auto take = [&](size_t bytes) {
+    const size_t here = at;
+    at += (bytes + kAlign - 1) / kAlign * kAlign;
+    return here;
+  };
+  const bool fp8 = l->recipe == B200MOE_RECIPE_FP8_BLOCK, mx = l->recipe == B200MOE_RECIPE_MXFP4;
+  w.rows = take(R * H * (fp8 || mx ? 1 : 2));
+  w.row_scales = take(fp8 ? R * (H / 128) * 4 : (mx ? R * mx_pitch(H) : 0));
+  w.act = take(R * I * (fp8 || mx ? 1 : 2));
+  w.act_scales = take(fp8 ? R * (I / 128) * 4 : (mx ? R * mx_pitch(I) : 0));
+  w.out = take(R * H * 2);
+  w.counts = take(static_cast<size_t>(l->E) * 4);
+  w.row_map = take(R * 4);
+  w.total = at;
+  return w;
+}
+
+// Up to about one routed row per local expert the block-FP8 GEMMs run on the decode-regime
+// kernel (weights on the M side of the MMA, 32 tokens per tile): 4-6 % faster end to end on the
+// DeepSeek-V3 shape.  From a few rows per expert on, hot experts need several 32-token chunks
+// that each stream the weights again, and the 128-row-tile kernel wins.
+bool decode_regime(const b200moe_layer* l, const b200moe_layer_call* c) {
+  if (l->recipe != B200MOE_RECIPE_FP8_BLOCK || l->gated_act != B200MOE_ACT_SILU || l->clamp_limit > 0.0f ||
+      c->valid_tokens)
+    return false;
+  if (const char* forced = getenv("B200MOE_DECODE_PATH")) return forced[0] == '1' && forced[1] == 0;
+  return static_cast<int64_t>(c->T) * c->k <= l->E;
+}
+
+int gemm(const b200moe_layer* l, const b200moe_layer_call* c, const Workspace& w, uint8_t* ws, bool second,
+         bool decode, void* stream) {
+  const int64_t R = static_cast<int64_t>(c->T) * c->k;
+  void* A = ws + (second ? w.act : w.rows);
+  void* sa = ws + (second ? w.act_scales : w.row_scales);
+  void* D = ws + (second ? w.out : w.act);
+  void* sd = ws + w.act_scales;
+  const int32_t* counts = reinterpret_cast<const int32_t*>(ws + w.counts);
+  const int N = second ? l->H : 2 * l->I, K = second ? l->I : l->H;
+  if (l->recipe == B200MOE_RECIPE_MXFP4) {
+    b200moe_mx_gemm_args a{};
+    a.epilogue = second ? B200MOE_EPI_STORE : l->epilogue;
+    a.d_dtype = second ? c->out_dtype : B200MOE_E4M3;
+    a.A = A;
+    a.a_sf = reinterpret_cast<const uint8_t*>(sa);
+    a.a_sf_pitch = static_cast<int64_t>(mx_pitch(K));
+    a.B = second ? l->w2 : l->w13;
+    a.b_sf = reinterpret_cast<const uint8_t*>(second ? l->w2_scale : l->w13_scale);
+    a.bias = second ? l->w2_bias : l->w13_bias;
+    a.bias_dtype = second ? l->w2_bias_dtype : l->w13_bias_dtype;
+    a.D = D;
+    a.d_sf = second ? nullptr : reinterpret_cast<uint8_t*>(sd);
+    a.d_sf_pitch = second ? 0 : static_cast<int64_t>(mx_pitch(l->I));
+    a.rows_per_expert = counts;
+    a.R = R;
+    a.N = N;
+    a.K = K;
+    a.E = l->E;
+    a.alpha = l->alpha;
+    a.limit = l->limit;
+    return b200moe_grouped_gemm_mx(&a, stream);
+  }
+  const bool fp8 = l->recipe == B200MOE_RECIPE_FP8_BLOCK;
+  b200moe_gemm_args a{};
+  a.recipe = l->recipe;
+  a.epilogue = second ? B200MOE_EPI_STORE : l->epilogue;
+  a.a_dtype = fp8 ? B200MOE_E4M3 : c->out_dtype;
+  a.d_dtype = second || !fp8 ? c->out_dtype : B200MOE_E4M3;
+  a.A = A;
+  a.a_scale = fp8 ? reinterpret_cast<const float*>(sa) : nullptr;
+  a.B = second ? l->w2 : l->w13;
+  a.b_layout = l->b_layout;
+  a.b_scale = second ? l->w2_scale : l->w13_scale;
+  a.bias = second ? l->w2_bias : l->w13_bias;
+  a.bias_dtype = second ? l->w2_bias_dtype : l->w13_bias_dtype;
+  a.D = D;
+  a.d_scale = fp8 && !second ? reinterpret_cast<float*>(sd) : nullptr;
+  a.rows_per_expert = counts;
+  a.R = R;
+  a.N = N;
+  a.K = K;
+  a.E = l->E;
+  a.alpha = l->alpha;
+  a.limit = l->limit;
+  a.a_scale_layout = decode ? B200MOE_A_SCALE_ROW_MAJOR_DECODE : B200MOE_A_SCALE_ROW_MAJOR;
+  if (!second) {
+    a.gated_act = l->gated_act;
+    a.act_param0 = l->act_param0;
+    a.act_param1 = l->act_param1;
+    a.clamp_limit = l->clamp_limit;
+  }
+  a.scales_pow2 = l->scales_pow2 && !decode;
+  return b200moe_grouped_gemm(&a, nullptr, 0, stream);
+}
+
+}  // namespace
+}  // namespace b200moe
+
+using namespace b200moe;
+
+extern "C" size_t b200moe_layer_workspace_bytes(const b200moe_layer* l, const b200moe_layer_call* c) {
+  if (!l || !c || c->T < 0 || c->k <= 0) return 0;
+  return carve(l, c).total;
+}
+
+extern "C" int b200moe_layer_forward(const b200moe_layer* l, const b200moe_layer_call* c, void* workspace,
+                                     size_t workspace_bytes, void* stream) {
+  if (!l || !c || c->T < 0 || c->k <= 0 || c->k > 64 || l->E <= 0 || l->H <= 0 || l->I <= 0)
+    return B200MOE_INVALID_ARG;
+  if (c->T == 0) return B200MOE_OK;
+  if (!c->x || !c->topk_weights || !c->topk_ids || !c->out || !is_index_dtype(c->ids_dtype)) return B200MOE_INVALID_ARG;
+  const bool fp8 = l->recipe == B200MOE_RECIPE_FP8_BLOCK, mx = l->recipe == B200MOE_RECIPE_MXFP4;
+  if (!fp8 && !mx && l->recipe != B200MOE_RECIPE_BF16) return B200MOE_UNSUPPORTED;
+  const bool x16 = c->x_dtype == B200MOE_BF16 || c->x_dtype == B200MOE_F16;
+  const bool quantised = c->x_dtype == B200MOE_E4M3;
+  if (quantised ? !((fp8 || mx) && c->x_scale) : !x16) return B200MOE_UNSUPPORTED;
+  if (!fp8 && !mx && c->x_dtype != c->out_dtype) return B200MOE_UNSUPPORTED;
+  if (c->out_dtype != B200MOE_BF16 && c->out_dtype != B200MOE_F16) return B200MOE_UNSUPPORTED;
+  if ((fp8 && (l->H % 128 || l->I % 128)) || (mx && (l->H % 64 || l->I % 64)) || l->H % 8) return B200MOE_UNSUPPORTED;
+  const Workspace w = carve(l, c);
+  if (!workspace || workspace_bytes < w.total) return B200MOE_WORKSPACE_TOO_SMALL;
+  uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
+  int32_t* row_map = reinterpret_cast<int32_t*>(ws + w.row_map);
+  int rc = B200MOE_OK;
+  if (c->stages & B200MOE_LAYER_PERMUTE) {
+    PermuteRows p{};
+    p.src = c->x;
+    p.src_scales = quantised ? c->x_scale : nullptr;
+    p.src_dtype = c->x_dtype;
+    p.mode = quantised || !(fp8 || mx) ? ROW_COPY : (fp8 ? ROW_QUANT_FP8 : ROW_QUANT_MX);
+    p.pow2_scales = l->scales_pow2;
+    p.row_bytes = static_cast<int64_t>(l->H) * (quantised ? 1 : 2);
+    p.scale_row_bytes = fp8 ? static_cast<int64_t>(l->H / 128) * 4 : (mx ? static_cast<int64_t>(mx_pitch(l->H)) : 0);
+    p.dst = ws + w.rows;
+    p.dst_scales = ws + w.row_scales;
+    p.ids = c->topk_ids;
+    p.ids_dtype = c->ids_dtype;
+    p.expert_map = c->expert_map;
+    p.T = c->T;
+    p.k = c->k;
+    p.total_experts = c->total_experts;
+    p.local_experts = l->E;
+    p.rows_per_expert = reinterpret_cast<int32_t*>(ws + w.counts);
+    p.accumulate = 0;
+    p.row_map = row_map;
+    rc = permute_rows(p, as_stream(stream));
+  }
+  const bool decode = decode_regime(l, c);
+  if (rc == B200MOE_OK && (c->stages & B200MOE_LAYER_GEMM1)) rc = gemm(l, c, w, ws, false, decode, stream);
+  if (rc == B200MOE_OK && (c->stages & B200MOE_LAYER_GEMM2)) rc = gemm(l, c, w, ws, true, decode, stream);
+  if (rc == B200MOE_OK && (c->stages & B200MOE_LAYER_COMBINE)) {
+    if (c->shared)
+      rc = b200moe_moe_gather_add(c->out, ws + w.out, c->out_dtype, c->topk_weights, row_map, c->shared, c->T, c->k,
+                                  l->H, stream);
+    else if (c->valid_tokens)
+      rc = b200moe_moe_gather_bounded(c->out, ws + w.out, c->out_dtype, c->topk_weights, row_map, c->valid_tokens,
+                                      c->T, c->k, l->H, stream);
+    else
+      rc = b200moe_moe_gather(c->out, ws + w.out, c->out_dtype, c->topk_weights, row_map, c->T, c->k, l->H, stream);
+  }
+  return rc;
+}

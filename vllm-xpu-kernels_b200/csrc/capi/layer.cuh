@@ -1,0 +1,36 @@
+// Internal entry shared by remap_hidden_states and the whole-layer call.
+#pragma once
+
+#include "common.cuh"
+
+namespace b200moe {
+
+// What happens to a row on its way to its permuted places.
+enum : int {
+  ROW_COPY = 0,      // copied as it is (with its row of scales, if it has one)
+  ROW_QUANT_FP8 = 1, // 16-bit row -> e4m3 + one f32 scale per 128 columns
+  ROW_QUANT_MX = 2   // 16-bit row -> e4m3 + one e8m0 byte per 32 columns
+};
+
+struct PermuteRows {
+  const void* src;            // [T, row_bytes]; null: grouping only
+  const void* src_scales;     // ROW_COPY: [T, scale_row_bytes] or null
+  int src_dtype;              // BF16 / F16 (ROW_QUANT_*)
+  int mode;
+  int pow2_scales;            // ROW_QUANT_FP8: scales rounded up to powers of two
+  int64_t row_bytes;          // of a source row, a multiple of 16
+  int64_t scale_row_bytes;    // of a row of (destination) scales
+  void* dst;                  // [T*k, row_bytes] or, quantised, [T*k, row_bytes / 2]
+  void* dst_scales;
+  const void* ids;
+  int ids_dtype;
+  const int32_t* expert_map;
+  int T, k, total_experts, local_experts;
+  int32_t* rows_per_expert;
+  int accumulate;             // rows_per_expert is added to instead of written
+  int32_t* row_map;           // [T, k]
+};
+
+int permute_rows(const PermuteRows& p, cudaStream_t st);
+
+}  // namespace b200moe

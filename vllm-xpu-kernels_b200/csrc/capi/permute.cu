@@ -2,22 +2,21 @@
 //
 // Both permutations are one stable counting sort of the flat (token, slot)
 // indices by expert, done with integers only so the result is reproducible and
-// equal to what a stable sort gives:
-//   1. count   — each CTA histograms a contiguous chunk of flat indices into
-//                 shared memory and writes its row of per-CTA counts;
-//   2. scan    — one CTA turns the [n_cta, E] counts into, for every
-//                 (cta, expert), the output position of that CTA's first
-//                 element of that expert (expert starts padded to the block
-//                 size for align), and writes the per-expert results;
-//   3. place   — each CTA walks its chunk again in index order; an element's
-//                 rank among equal experts comes from a warp match plus
-//                 per-warp running offsets, never from atomics.
-// Inputs that fit one chunk take a single fused launch.
+// equal to what a stable sort gives: every warp histograms a contiguous run of
+// indices into shared memory, counts are prefix-summed over warps (and over the
+// CTAs of a cluster), then every warp walks its run again in index order; an
+// element's rank among equal experts comes from a warp match plus the warp's
+// running offsets, never from atomics.
+//   numel <= 2048: one CTA;
+//   larger:        one cluster of eight CTAs that exchange their counts through
+//                  distributed shared memory -- one launch, no workspace;
+//   the layer's own few-token path: every CTA of the row kernel groups for itself.
+#include <cooperative_groups.h>
 #include <stdio.h>
 
-#include <mutex>
-
 #include "common.cuh"
+#include "layer.cuh"
+#include "quant_math.cuh"
 
 namespace b200moe {
 namespace {
@@ -81,6 +80,7 @@ __device__ __forceinline__ void chunk_place(const GroupParams& p, int64_t base,
   for (int e = threadIdx.x; e < p.num_keys * kWarps; e += kThreads) warp_off[e] = 0;
   __syncthreads();
   int keys[kPerWarp / 32];
+  const int64_t left = p.numel - base - warp * kPerWarp;   // indices from this warp's first one on
 #pragma unroll
   for (int s = 0; s < kPerWarp / 32; ++s) {
     const int64_t idx = base + warp * kPerWarp + s * 32 + lane;
@@ -102,6 +102,7 @@ __device__ __forceinline__ void chunk_place(const GroupParams& p, int64_t base,
   int* mine = warp_off + warp * p.num_keys;
 #pragma unroll
   for (int s = 0; s < kPerWarp / 32; ++s) {
+    if (s * 32 >= left) break;   // same for the whole warp
     const int key = keys[s];
     const unsigned peers = __match_any_sync(0xffffffffu, key);
     if (key >= 0) {
@@ -113,13 +114,6 @@ __device__ __forceinline__ void chunk_place(const GroupParams& p, int64_t base,
     if (key >= 0 && lane == (31 - __clz(peers))) mine[key] += __popc(peers);
     __syncwarp();
   }
-}
-
-__global__ void __launch_bounds__(kThreads) count_kernel(GroupParams p, int* __restrict__ counts) {
-  extern __shared__ int smem[];
-  chunk_histogram(p, static_cast<int64_t>(blockIdx.x) * kChunk, smem);
-  for (int e = threadIdx.x; e < p.num_keys; e += kThreads)
-    counts[static_cast<int64_t>(blockIdx.x) * p.num_keys + e] = smem[e];
 }
 
 // Per-key totals -> padded starts (exclusive scan over keys, any num_keys <=
@@ -186,78 +180,17 @@ __device__ __forceinline__ void write_align_meta(const AlignOut& o, int num_keys
   if (threadIdx.x == 0) o.total[0] = grand_total;
 }
 
-// counts [n_cta, E] -> in place: position of each CTA's first element per key.
-__global__ void __launch_bounds__(kThreads) scan_kernel(GroupParams p, int n_cta,
-                                                        int* __restrict__ counts, AlignOut ao,
-                                                        int32_t* __restrict__ rows_per_key) {
-  __shared__ int total[kMaxExperts];
-  __shared__ int start[kMaxExperts];
-  __shared__ int grand;
-  for (int e = threadIdx.x; e < p.num_keys; e += kThreads) {
-    int run = 0;
-    for (int c = 0; c < n_cta; ++c) run += counts[static_cast<int64_t>(c) * p.num_keys + e];
-    total[e] = run;
-  }
-  __syncthreads();
-  scan_keys(p.num_keys, p.block_size, total, start, &grand);
-  for (int e = threadIdx.x; e < p.num_keys; e += kThreads) {
-    int run = start[e];
-    for (int c = 0; c < n_cta; ++c) {
-      const int64_t at = static_cast<int64_t>(c) * p.num_keys + e;
-      const int cnt = counts[at];
-      counts[at] = run;
-      run += cnt;
-    }
-    if (rows_per_key) rows_per_key[e] += total[e];
-  }
-  if (ao.sorted_ids) write_align_meta(ao, p.num_keys, p.block_size, total, start, grand);
-}
-
-__global__ void fill_kernel(int32_t* __restrict__ dst, int64_t n, int32_t value) {
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    dst[i] = value;
-}
-
-__global__ void __launch_bounds__(kThreads) place_align_kernel(GroupParams p,
-                                                               const int* __restrict__ bases,
-                                                               AlignOut ao) {
-  extern __shared__ int smem[];
-  int* cta_base = smem;
-  int* warp_off = smem + p.num_keys;
-  for (int e = threadIdx.x; e < p.num_keys; e += kThreads)
-    cta_base[e] = bases[static_cast<int64_t>(blockIdx.x) * p.num_keys + e];
-  __syncthreads();
-  chunk_place(p, static_cast<int64_t>(blockIdx.x) * kChunk, cta_base, warp_off,
-              [&](int64_t idx, int, int pos) {
-                if (pos < ao.sorted_capacity) ao.sorted_ids[pos] = static_cast<int32_t>(idx);
-              });
-}
-
-__global__ void __launch_bounds__(kThreads) place_remap_kernel(GroupParams p,
-                                                               const int* __restrict__ bases,
-                                                               int32_t* __restrict__ row_map) {
-  extern __shared__ int smem[];
-  int* cta_base = smem;
-  int* warp_off = smem + p.num_keys;
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * kChunk;
-  for (int e = threadIdx.x; e < p.num_keys; e += kThreads)
-    cta_base[e] = bases[static_cast<int64_t>(blockIdx.x) * p.num_keys + e];
-  for (int i = threadIdx.x; i < kChunk; i += kThreads)
-    if (base + i < p.numel) row_map[base + i] = -1;
-  __syncthreads();
-  chunk_place(p, base, cta_base, warp_off,
-              [&](int64_t idx, int, int pos) { row_map[idx] = pos; });
-}
-
 // Whole permutation in one CTA when numel <= kChunk.
 __global__ void __launch_bounds__(kThreads) fused_small_kernel(GroupParams p, AlignOut ao,
                                                                int32_t* __restrict__ rows_per_key,
+                                                               int accumulate,
                                                                int32_t* __restrict__ row_map) {
   extern __shared__ int smem[];
   __shared__ int total[kMaxExperts];
   __shared__ int start[kMaxExperts];
   __shared__ int grand;
+  pdl_wait();
+  pdl_trigger();
   int* warp_off = smem;
   chunk_histogram(p, 0, total);
   scan_keys(p.num_keys, p.block_size, total, start, &grand);
@@ -267,7 +200,8 @@ __global__ void __launch_bounds__(kThreads) fused_small_kernel(GroupParams p, Al
       ao.sorted_ids[i] = static_cast<int32_t>(p.numel);
   }
   if (rows_per_key)
-    for (int e = threadIdx.x; e < p.num_keys; e += kThreads) rows_per_key[e] += total[e];
+    for (int e = threadIdx.x; e < p.num_keys; e += kThreads)
+      rows_per_key[e] = (accumulate ? rows_per_key[e] : 0) + total[e];
   if (row_map)
     for (int i = threadIdx.x; i < p.numel; i += kThreads) row_map[i] = -1;
   __syncthreads();
@@ -278,6 +212,154 @@ __global__ void __launch_bounds__(kThreads) fused_small_kernel(GroupParams p, Al
       row_map[idx] = pos;
     }
   });
+}
+
+// The same for any number of indices: one cluster of kGroupCtas CTAs.  Bound by latency, not
+// by bytes (0.5 MB of indices at 16384 tokens x 8): what counts is the number of dependent
+// steps.  Three launches (count, scan over per-CTA counts, place) took 16 us at 18 k indices
+// and 26 us at 131 k; here the counts never leave shared memory.
+constexpr int kGroupCtas = 8;
+constexpr int kGroupThreads = 512;
+constexpr int kGroupWarps = kGroupThreads / 32;
+
+__global__ void __cluster_dims__(kGroupCtas, 1, 1) __launch_bounds__(kGroupThreads)
+group_cluster_kernel(GroupParams p, AlignOut ao, int32_t* __restrict__ rows_per_key, int accumulate,
+                     int32_t* __restrict__ row_map) {
+  namespace cg = cooperative_groups;
+  extern __shared__ int smem[];
+  __shared__ int total[kMaxExperts];   // this CTA's counts; read by the other CTAs
+  __shared__ int grand_of[kMaxExperts];
+  __shared__ int start[kMaxExperts];
+  __shared__ int warp_sums[kGroupWarps];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = static_cast<int>(cluster.block_rank());
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int K = p.num_keys;
+  int* mine = smem + warp * K;   // this warp's counts, then its running positions
+  pdl_wait();
+  pdl_trigger();
+  for (int e = threadIdx.x; e < K * kGroupWarps; e += kGroupThreads) smem[e] = 0;
+  __syncthreads();
+  const int64_t per_warp = (p.numel + kGroupCtas * kGroupThreads - 1) / (kGroupCtas * kGroupThreads) * 32;
+  const int64_t lo = (static_cast<int64_t>(rank) * kGroupWarps + warp) * per_warp;
+  const int64_t hi = lo + per_warp < p.numel ? lo + per_warp : p.numel;
+  constexpr int kHeld = 16;      // keys kept in registers between the two walks
+  int keys[kHeld];
+#pragma unroll
+  for (int s = 0; s < kHeld; ++s) {
+    const int64_t idx = lo + s * 32 + lane;
+    keys[s] = idx < hi ? key_of(p, idx) : -1;
+  }
+#pragma unroll
+  for (int s = 0; s < kHeld; ++s)
+    if (keys[s] >= 0) atomicAdd(&mine[keys[s]], 1);
+  for (int64_t idx = lo + kHeld * 32 + lane; idx < hi; idx += 32) {
+    const int key = key_of(p, idx);
+    if (key >= 0) atomicAdd(&mine[key], 1);
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < K; e += kGroupThreads) {
+    int run = 0;
+    for (int w = 0; w < kGroupWarps; ++w) {
+      const int c = smem[w * K + e];
+      smem[w * K + e] = run;
+      run += c;
+    }
+    total[e] = run;
+  }
+  cluster.sync();
+  int before[2] = {0, 0};   // of keys threadIdx.x and threadIdx.x + 512: counts of the CTAs before this one
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int e = threadIdx.x + j * kGroupThreads;
+    if (e >= K) break;
+    int sum = 0;
+#pragma unroll
+    for (int c = 0; c < kGroupCtas; ++c) {
+      const int v = cluster.map_shared_rank(total, c)[e];
+      if (c < rank) before[j] += v;
+      sum += v;
+    }
+    grand_of[e] = sum;
+  }
+  __syncthreads();
+  // exclusive scan of the padded counts over the keys, two neighbouring keys per thread
+  {
+    int v[2], local = 0;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int e = threadIdx.x * 2 + j;
+      v[j] = e < K ? (grand_of[e] + p.block_size - 1) / p.block_size * p.block_size : 0;
+      local += v[j];
+    }
+    int incl = local;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += o;
+    }
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    int base = 0;
+    for (int w = 0; w < warp; ++w) base += warp_sums[w];
+    const int e0 = threadIdx.x * 2;
+    if (e0 < K) start[e0] = base + incl - local;
+    if (e0 + 1 < K) start[e0 + 1] = base + incl - v[1];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int e = threadIdx.x + j * kGroupThreads;
+    if (e >= K) break;
+    const int add = start[e] + before[j];
+    for (int w = 0; w < kGroupWarps; ++w) smem[w * K + e] += add;
+    if (rank == 0 && rows_per_key) rows_per_key[e] = (accumulate ? rows_per_key[e] : 0) + grand_of[e];
+  }
+  __syncthreads();
+  auto place = [&](int key, int64_t idx) {
+    const unsigned peers = __match_any_sync(0xffffffffu, key);
+    if (key >= 0) {
+      const int pos = mine[key] + __popc(peers & ((1u << lane) - 1u));
+      if (ao.sorted_ids) {
+        if (pos < ao.sorted_capacity) ao.sorted_ids[pos] = static_cast<int32_t>(idx);
+      } else {
+        row_map[idx] = pos;
+      }
+    } else if (row_map && idx < hi) {
+      row_map[idx] = -1;
+    }
+    __syncwarp();
+    if (key >= 0 && lane == (31 - __clz(peers))) mine[key] += __popc(peers);
+    __syncwarp();
+  };
+#pragma unroll
+  for (int s = 0; s < kHeld; ++s) {
+    if (lo + s * 32 >= hi) break;
+    place(keys[s], lo + s * 32 + lane);
+  }
+  for (int64_t i = lo + kHeld * 32; i < hi; i += 32)
+    place(i + lane < hi ? key_of(p, i + lane) : -1, i + lane);
+  if (ao.sorted_ids) {
+    // one warp of the cluster per key: its block labels and the padding behind its run
+    const int last = K - 1;
+    const int all = start[last] + (grand_of[last] + p.block_size - 1) / p.block_size * p.block_size;
+    const int32_t pad = static_cast<int32_t>(p.numel);
+    for (int e = rank * kGroupWarps + warp; e < K; e += kGroupCtas * kGroupWarps) {
+      const int n = grand_of[e];
+      const int end = start[e] + (n + p.block_size - 1) / p.block_size * p.block_size;
+      for (int i = start[e] + n + lane; i < end; i += 32)
+        if (i < ao.sorted_capacity) ao.sorted_ids[i] = pad;
+      const int label = ao.expert_map ? ao.expert_map[e] : e;
+      for (int b = start[e] / p.block_size + lane; b < end / p.block_size; b += 32)
+        if (b < ao.blocks_capacity) ao.expert_ids[b] = label;
+    }
+    const int64_t gid = rank * kGroupThreads + threadIdx.x;
+    for (int64_t i = all + gid; i < ao.sorted_capacity; i += kGroupCtas * kGroupThreads) ao.sorted_ids[i] = pad;
+    for (int64_t b = all / p.block_size + gid; b < ao.blocks_capacity; b += kGroupCtas * kGroupThreads)
+      ao.expert_ids[b] = ao.tail_label;
+    if (gid == 0) ao.total[0] = all;
+  }
+  cluster.sync();   // no CTA leaves while another may still read its counts
 }
 
 // Multi-LoRA alignment: CTA x handles the adapter slot lora_ids[x] and builds that slot's
@@ -324,70 +406,171 @@ __global__ void __launch_bounds__(kThreads) lora_align_kernel(
   }
 }
 
-int run_grouping(const GroupParams& p, const AlignOut& ao, int32_t* rows_per_key,
-                 int32_t* row_map, void* ws, size_t ws_bytes, cudaStream_t st) {
+int run_grouping(const GroupParams& p, const AlignOut& ao, int32_t* rows_per_key, int accumulate,
+                 int32_t* row_map, cudaStream_t st) {
   if (p.num_keys > kMaxExperts) return B200MOE_UNSUPPORTED;
-  const int64_t n_cta64 = (p.numel + kChunk - 1) / kChunk;
-  const size_t place_smem = static_cast<size_t>(p.num_keys) * (1 + kWarps) * sizeof(int);
-  if (n_cta64 <= 1) {
-    fused_small_kernel<<<1, kThreads, p.num_keys * kWarps * sizeof(int), st>>>(p, ao, rows_per_key,
-                                                                              row_map);
-    return launch_status("fused_small_kernel");
-  }
-  const int n_cta = static_cast<int>(n_cta64);
-  const size_t need = static_cast<size_t>(n_cta) * p.num_keys * sizeof(int);
-  if (!ws || ws_bytes < need) return B200MOE_WORKSPACE_TOO_SMALL;
-  int* counts = reinterpret_cast<int*>(ws);
-  if (ao.sorted_ids) {
-    const int blocks = static_cast<int>((ao.sorted_capacity + 4095) / 4096);
-    fill_kernel<<<blocks < 592 ? blocks : 592, 256, 0, st>>>(ao.sorted_ids, ao.sorted_capacity,
-                                                             static_cast<int32_t>(p.numel));
-  }
-  count_kernel<<<n_cta, kThreads, p.num_keys * sizeof(int), st>>>(p, counts);
-  scan_kernel<<<1, kThreads, 0, st>>>(p, n_cta, counts, ao, rows_per_key);
-  if (ao.sorted_ids)
-    place_align_kernel<<<n_cta, kThreads, place_smem, st>>>(p, counts, ao);
-  else
-    place_remap_kernel<<<n_cta, kThreads, place_smem, st>>>(p, counts, row_map);
-  for (int i = 0; i < (ao.sorted_ids ? 3 : 2); ++i) count_launch();  // launch_status counts the last one
-  return launch_status("stable grouping");
+  if (p.numel <= kChunk)
+    return launch_pdl("fused_small_kernel", fused_small_kernel, dim3(1), dim3(kThreads),
+                      p.num_keys * kWarps * sizeof(int), st, 1, p, ao, rows_per_key, accumulate, row_map);
+  struct Tag {};
+  const int rc = ensure_dynamic_smem<Tag>(group_cluster_kernel, kMaxExperts * kGroupWarps * sizeof(int),
+                                          "cudaFuncSetAttribute (grouping)");
+  if (rc != B200MOE_OK) return rc;
+  return launch_pdl("group_cluster_kernel", group_cluster_kernel, dim3(kGroupCtas), dim3(kGroupThreads),
+                    static_cast<size_t>(p.num_keys) * kGroupWarps * sizeof(int), st, 1, p, ao, rows_per_key,
+                    accumulate, row_map);
 }
 
-// ---- row copy of remap_hidden_states ------------------------------------------
+// ---- rows to their permuted places ---------------------------------------------
 
-// One CTA per token: the row is read once and written to each of its k
-// permuted positions in 16-byte pieces.
-__global__ void __launch_bounds__(256) copy_rows_kernel(
-    const uint4* __restrict__ src, const uint8_t* __restrict__ src_scale,
-    uint4* __restrict__ dst, uint8_t* __restrict__ dst_scale, int64_t row_vecs,
-    int64_t scale_row_bytes, const int32_t* __restrict__ row_map, int k) {
+// One CTA per token (and per part of the row when tokens are few): the row is read once,
+// quantised if asked, and written to each of its permuted positions.  Streaming: reads
+// T * row_bytes, writes T * k * (row or half a row); what the separate passes cost was one more
+// read and write of every row.  A token without a local expert is not read at all.
+//
+// GROUP (numel <= 2048): no grouping launch before it.  Every CTA histograms all ids into shared
+// memory and ranks its own k entries by counting equal ids with a lower index: 2048 comparisons
+// per entry spread over 256 threads, less than the launch and the round trip of a row map.
+constexpr int kMaxRowTopK = 64;
+
+struct RowsParams {
+  const uint8_t* src;
+  const uint8_t* src_scale;
+  uint8_t* dst;
+  uint8_t* dst_scale;
+  int row_vecs;             // 16-byte pieces of a source row
+  int vecs_per_part;
+  int64_t scale_row_bytes;
+  int k;
+  int pow2;
+  int32_t* row_map;
+  int32_t* rows_per_key;
+  int accumulate;
+};
+
+template <typename T, int MODE, bool GROUP>
+__global__ void __launch_bounds__(kThreads) rows_kernel(GroupParams g, RowsParams p) {
+  __shared__ int rows[kMaxRowTopK];
+  __shared__ int hist[GROUP ? kMaxExperts : 1];
+  __shared__ int own_key[GROUP ? kMaxRowTopK : 1], own_rank[GROUP ? kMaxRowTopK : 1];
   const int64_t t = blockIdx.x;
-  __shared__ int rows[64];
-  for (int j = threadIdx.x; j < k; j += blockDim.x) rows[j] = row_map[t * k + j];
-  __syncthreads();
-  const uint4* s = src + t * row_vecs;
-  for (int64_t v = threadIdx.x; v < row_vecs; v += blockDim.x) {
-    const uint4 val = s[v];
+  const int k = p.k;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int v0 = blockIdx.y * p.vecs_per_part;
+  const int v1 = min(v0 + p.vecs_per_part, p.row_vecs);
+  const uint4* src = reinterpret_cast<const uint4*>(p.src) + t * p.row_vecs;
+  pdl_wait();
+  pdl_trigger();
+  uint4 val = make_uint4(0, 0, 0, 0);
+  if constexpr (GROUP) {
+    if (p.src && v0 + static_cast<int>(threadIdx.x) < v1) val = src[v0 + threadIdx.x];  // in flight while grouping
+    constexpr int kSteps = kChunk / kThreads;
+    int keys[kSteps];
+#pragma unroll
+    for (int s = 0; s < kSteps; ++s) {
+      const int idx = s * kThreads + threadIdx.x;
+      keys[s] = idx < g.numel ? key_of(g, idx) : -1;
+    }
+    for (int e = threadIdx.x; e < g.num_keys; e += kThreads) hist[e] = 0;
+    if (threadIdx.x < k) {
+      own_key[threadIdx.x] = key_of(g, t * k + threadIdx.x);
+      own_rank[threadIdx.x] = 0;
+    }
+    __syncthreads();
+    const int first = static_cast<int>(t) * k;
+#pragma unroll
+    for (int s = 0; s < kSteps; ++s)
+      if (keys[s] >= 0) atomicAdd(&hist[keys[s]], 1);
     for (int j = 0; j < k; ++j) {
-      const int r = rows[j];
-      if (r >= 0) dst[static_cast<int64_t>(r) * row_vecs + v] = val;
+      const int want = own_key[j];
+      int n = 0;
+#pragma unroll
+      for (int s = 0; s < kSteps; ++s)
+        n += (keys[s] == want && s * kThreads + static_cast<int>(threadIdx.x) < first + j) ? 1 : 0;
+      if (__any_sync(0xffffffffu, n)) {
+        n = __reduce_add_sync(0xffffffffu, n);
+        if (lane == 0) atomicAdd(&own_rank[j], n);
+      }
+    }
+    __syncthreads();
+    for (int j = warp; j < k; j += kWarps) {
+      const int key = own_key[j];
+      int n = 0;
+      for (int e = lane; e < key; e += 32) n += hist[e];
+      n = __reduce_add_sync(0xffffffffu, n);
+      if (lane == 0) {
+        const int pos = key < 0 ? -1 : n + own_rank[j];
+        rows[j] = pos;
+        if (blockIdx.y == 0) p.row_map[t * k + j] = pos;
+      }
+    }
+    if (t == 0 && blockIdx.y == 0 && p.rows_per_key)
+      for (int e = threadIdx.x; e < g.num_keys; e += kThreads)
+        p.rows_per_key[e] = (p.accumulate ? p.rows_per_key[e] : 0) + hist[e];
+    if (!p.src) return;
+  } else {
+    for (int j = threadIdx.x; j < k; j += kThreads) rows[j] = p.row_map[t * k + j];
+  }
+  __syncthreads();
+  int top = -1;
+  for (int j = 0; j < k; ++j) top = max(top, rows[j]);
+  if (top < 0) return;   // no local expert
+  for (int base = v0; base < v1; base += kThreads) {
+    const int v = base + threadIdx.x;
+    const bool live = v < v1;
+    if ((!GROUP || base != v0) && live) val = src[v];
+    if constexpr (MODE == ROW_COPY) {
+      if (live)
+        for (int j = 0; j < k; ++j) {
+          const int r = rows[j];
+          if (r >= 0) reinterpret_cast<uint4*>(p.dst)[static_cast<int64_t>(r) * p.row_vecs + v] = val;
+        }
+    } else {
+      float x[8];
+      const T* e = reinterpret_cast<const T*>(&val);
+      float amax = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        x[i] = live ? Elem<T>::to_f32(e[i]) : 0.f;
+        amax = fmaxf(amax, fabsf(x[i]));
+      }
+      uint2 q;
+      float s = 0.f;
+      uint32_t exponent = 0;
+      if constexpr (MODE == ROW_QUANT_FP8) {
+        amax = seg_max<16>(amax);
+        s = fp8_group_scale(amax, 1e-10f, 448.0f, p.pow2 != 0);
+        q = quantise8_e4m3(x, 1.0f / s);
+      } else {
+        amax = seg_max<4>(amax);
+        exponent = mxfp8_scale_exponent(amax);
+        q = quantise8_e4m3(x, 1.0f / __uint_as_float(exponent << 23));
+      }
+      if (!live) continue;
+      for (int j = 0; j < k; ++j) {
+        const int64_t r = rows[j];
+        if (r < 0) continue;
+        reinterpret_cast<uint2*>(p.dst)[r * p.row_vecs + v] = q;
+        if constexpr (MODE == ROW_QUANT_FP8) {
+          if ((threadIdx.x & 15) == 0) reinterpret_cast<float*>(p.dst_scale + r * p.scale_row_bytes)[v >> 4] = s;
+        } else {
+          if ((threadIdx.x & 3) == 0) p.dst_scale[r * p.scale_row_bytes + (v >> 2)] = static_cast<uint8_t>(exponent);
+        }
+      }
     }
   }
-  if (src_scale) {
-    const uint8_t* ss = src_scale + t * scale_row_bytes;
-    if ((scale_row_bytes & 3) == 0) {
-      for (int64_t v = threadIdx.x; v < scale_row_bytes / 4; v += blockDim.x) {
-        const uint32_t val = reinterpret_cast<const uint32_t*>(ss)[v];
+  if (MODE == ROW_COPY && p.src_scale && blockIdx.y == 0) {
+    const uint8_t* ss = p.src_scale + t * p.scale_row_bytes;
+    if ((p.scale_row_bytes & 3) == 0) {
+      for (int v = threadIdx.x; v < p.scale_row_bytes / 4; v += kThreads) {
+        const uint32_t w = reinterpret_cast<const uint32_t*>(ss)[v];
         for (int j = 0; j < k; ++j)
-          if (rows[j] >= 0)
-            reinterpret_cast<uint32_t*>(dst_scale + static_cast<int64_t>(rows[j]) * scale_row_bytes)[v] = val;
+          if (rows[j] >= 0) reinterpret_cast<uint32_t*>(p.dst_scale + static_cast<int64_t>(rows[j]) * p.scale_row_bytes)[v] = w;
       }
     } else {
-      for (int64_t v = threadIdx.x; v < scale_row_bytes; v += blockDim.x) {
-        const uint8_t val = ss[v];
+      for (int v = threadIdx.x; v < p.scale_row_bytes; v += kThreads)
         for (int j = 0; j < k; ++j)
-          if (rows[j] >= 0) dst_scale[static_cast<int64_t>(rows[j]) * scale_row_bytes + v] = val;
-      }
+          if (rows[j] >= 0) p.dst_scale[static_cast<int64_t>(rows[j]) * p.scale_row_bytes + v] = ss[v];
     }
   }
 }
@@ -400,13 +583,55 @@ __global__ void init_expert_map_kernel(int32_t* map, int num_local, int ep_rank,
 }
 
 }  // namespace
+
+int permute_rows(const PermuteRows& a, cudaStream_t st) {
+  if (a.T == 0) return B200MOE_OK;
+  GroupParams g{a.ids, a.ids_dtype, static_cast<int64_t>(a.T) * a.k, a.local_experts,
+                a.expert_map ? a.total_experts : a.local_experts, a.expert_map, 0, 1};
+  const bool inside = g.numel <= kChunk && a.local_experts <= kMaxExperts;
+  if (!inside) {
+    AlignOut none{nullptr, 0, nullptr, 0, nullptr, nullptr};
+    const int rc = run_grouping(g, none, a.rows_per_expert, a.accumulate, a.row_map, st);
+    if (rc != B200MOE_OK || !a.src) return rc;
+  }
+  RowsParams p{reinterpret_cast<const uint8_t*>(a.src), reinterpret_cast<const uint8_t*>(a.src_scales),
+               reinterpret_cast<uint8_t*>(a.dst), reinterpret_cast<uint8_t*>(a.dst_scales),
+               static_cast<int>(a.row_bytes / 16), 0, a.scale_row_bytes, a.k, a.pow2_scales, a.row_map,
+               a.rows_per_expert, a.accumulate};
+  // Few tokens: split the row so that about two CTAs per SM have something to do.  Parts are
+  // whole quantisation groups (16 pieces = 128 columns).
+  int parts = (2 * kNumSMs + a.T - 1) / a.T;
+  const int most = (p.row_vecs + kThreads / 2 - 1) / (kThreads / 2);
+  if (parts > most) parts = most;
+  if (parts < 1 || !a.src) parts = 1;
+  p.vecs_per_part = ((p.row_vecs + parts - 1) / parts + 15) / 16 * 16;
+  parts = p.vecs_per_part ? (p.row_vecs + p.vecs_per_part - 1) / p.vecs_per_part : 1;
+  if (parts < 1) parts = 1;
+  const dim3 grid(a.T, parts);
+  auto go = [&](auto kernel) {
+    return launch_pdl("rows_kernel", kernel, grid, dim3(kThreads), 0, st, 1, g, p);
+  };
+  const bool f16 = a.src_dtype == B200MOE_F16;
+  if (a.mode == ROW_QUANT_FP8) {
+    if (inside) return f16 ? go(rows_kernel<__half, ROW_QUANT_FP8, true>) : go(rows_kernel<__nv_bfloat16, ROW_QUANT_FP8, true>);
+    return f16 ? go(rows_kernel<__half, ROW_QUANT_FP8, false>) : go(rows_kernel<__nv_bfloat16, ROW_QUANT_FP8, false>);
+  }
+  if (a.mode == ROW_QUANT_MX) {
+    if (inside) return f16 ? go(rows_kernel<__half, ROW_QUANT_MX, true>) : go(rows_kernel<__nv_bfloat16, ROW_QUANT_MX, true>);
+    return f16 ? go(rows_kernel<__half, ROW_QUANT_MX, false>) : go(rows_kernel<__nv_bfloat16, ROW_QUANT_MX, false>);
+  }
+  return inside ? go(rows_kernel<uint8_t, ROW_COPY, true>) : go(rows_kernel<uint8_t, ROW_COPY, false>);
+}
+
 }  // namespace b200moe
 
 using namespace b200moe;
 
-size_t grouping_workspace(int64_t numel, int num_keys) {
-  const int64_t n_cta = (numel + kChunk - 1) / kChunk;
-  return n_cta <= 1 ? 0 : static_cast<size_t>(n_cta) * num_keys * sizeof(int);
+// The workspace of the grouping entry points is part of their contract (a count per 2048 indices
+// and expert); the counts now stay in shared memory and a null workspace is as good.
+static size_t grouping_workspace(int64_t numel, int num_keys) {
+  const int64_t chunks = (numel + kChunk - 1) / kChunk;
+  return chunks <= 1 ? 0 : static_cast<size_t>(chunks) * num_keys * sizeof(int);
 }
 
 extern "C" size_t b200moe_moe_align_block_size_workspace_bytes(int64_t numel, int num_experts) {
@@ -418,7 +643,7 @@ extern "C" int b200moe_moe_align_block_size(const void* topk_ids, int ids_dtype,
                                             const int32_t* expert_map, int32_t* sorted_token_ids,
                                             int64_t sorted_capacity, int32_t* expert_ids,
                                             int64_t blocks_capacity, int32_t* num_tokens_post_pad,
-                                            void* workspace, size_t workspace_bytes,
+                                            void* /*workspace*/, size_t /*workspace_bytes*/,
                                             void* stream) {
   if (numel < 0 || num_experts <= 0 || block_size <= 0 || !is_index_dtype(ids_dtype) ||
       !sorted_token_ids || !expert_ids || !num_tokens_post_pad || (numel > 0 && !topk_ids))
@@ -431,7 +656,7 @@ extern "C" int b200moe_moe_align_block_size(const void* topk_ids, int ids_dtype,
   GroupParams p{topk_ids, ids_dtype, numel, num_experts, num_experts, expert_map, 0, block_size};
   AlignOut ao{sorted_token_ids, sorted_capacity, expert_ids, blocks_capacity, num_tokens_post_pad,
               nullptr};
-  return run_grouping(p, ao, nullptr, nullptr, workspace, workspace_bytes, as_stream(stream));
+  return run_grouping(p, ao, nullptr, 0, nullptr, as_stream(stream));
 }
 
 extern "C" int b200moe_init_expert_map(int32_t* expert_map, int num_local_experts, int ep_rank,
@@ -454,70 +679,21 @@ extern "C" int b200moe_remap_hidden_states(const void* hidden, const void* scale
                                            int ids_dtype, const int32_t* expert_map, int T, int k,
                                            int total_experts, int local_experts,
                                            int32_t* rows_per_expert, int32_t* row_map,
-                                           void* workspace, size_t workspace_bytes,
+                                           void* /*workspace*/, size_t /*workspace_bytes*/,
                                            void* stream) {
-  if (T < 0 || k <= 0 || k > 64 || local_experts <= 0 || total_experts <= 0 ||
+  if (T < 0 || k <= 0 || k > kMaxRowTopK || local_experts <= 0 || total_experts <= 0 ||
       !is_index_dtype(ids_dtype) || !rows_per_expert || !row_map)
     return B200MOE_INVALID_ARG;
   if (row_bytes % 16 != 0) return B200MOE_INVALID_ARG;
   if (T == 0) return B200MOE_OK;
   if (!topk_ids || (hidden && !remapped) || (scales && !remapped_scales)) return B200MOE_INVALID_ARG;
-  cudaStream_t st = as_stream(stream);
-  GroupParams p{topk_ids, ids_dtype, static_cast<int64_t>(T) * k, local_experts,
-                expert_map ? total_experts : local_experts, expert_map, 0, 1};
-  AlignOut none{nullptr, 0, nullptr, 0, nullptr, nullptr};
-  int rc = run_grouping(p, none, rows_per_expert, row_map, workspace, workspace_bytes, st);
-  if (rc != B200MOE_OK) return rc;
-  if (hidden) {
-    copy_rows_kernel<<<T, 256, 0, st>>>(reinterpret_cast<const uint4*>(hidden),
-                                        reinterpret_cast<const uint8_t*>(scales),
-                                        reinterpret_cast<uint4*>(remapped),
-                                        reinterpret_cast<uint8_t*>(remapped_scales),
-                                        row_bytes / 16, scale_row_bytes, row_map, k);
-    rc = launch_status("copy_rows_kernel");
-  }
-  return rc;
+  if (local_experts > kMaxExperts) return B200MOE_UNSUPPORTED;
+  PermuteRows p{hidden, scales, B200MOE_BF16, ROW_COPY, 0, row_bytes, scale_row_bytes, remapped, remapped_scales,
+                topk_ids, ids_dtype, expert_map, T, k, total_experts, local_experts, rows_per_expert, 1, row_map};
+  return permute_rows(p, as_stream(stream));
 }
 
 // ---- moe_align_block_size for callers that cannot allocate ----------------------
-
-namespace b200moe {
-namespace {
-
-// Scratch of the allocation-free entry point: 64 Ki ints = 256 KiB of every GPU
-// that loads this library, held until the process exits.
-constexpr int kStaticScratchInts = 64 * 1024;
-static __device__ __align__(256) int g_align_static_scratch[kStaticScratchInts];
-
-constexpr int kMaxDevices = 64;
-
-// Device address of the array above on the current device.  In host code the
-// array's name is only a handle for the runtime, never a pointer a kernel could
-// use, so the address is looked up once per device (with that device current).
-int* static_scratch_on_current_device() {
-  static std::mutex mu;
-  static int* cached[kMaxDevices] = {};
-  int dev = -1;
-  cudaError_t err = cudaGetDevice(&dev);
-  if (err != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
-    set_last_error("moe_align_block_size_static: cudaGetDevice", err);
-    return nullptr;
-  }
-  std::lock_guard<std::mutex> lock(mu);
-  if (!cached[dev]) {
-    void* ptr = nullptr;
-    err = cudaGetSymbolAddress(&ptr, g_align_static_scratch);
-    if (err != cudaSuccess || !ptr) {
-      set_last_error("moe_align_block_size_static: cudaGetSymbolAddress", err);
-      return nullptr;
-    }
-    cached[dev] = static_cast<int*>(ptr);
-  }
-  return cached[dev];
-}
-
-}  // namespace
-}  // namespace b200moe
 
 extern "C" int b200moe_moe_align_block_size_static(const void* topk_ids, int ids_dtype,
                                                    int64_t numel, int num_experts, int block_size,
@@ -527,27 +703,21 @@ extern "C" int b200moe_moe_align_block_size_static(const void* topk_ids, int ids
                                                    int64_t blocks_capacity,
                                                    int32_t* num_tokens_post_pad, void* stream) {
   if (numel < 0 || num_experts <= 0) return B200MOE_INVALID_ARG;
-  const size_t need = grouping_workspace(numel, num_experts);
-  if (need > sizeof(int) * static_cast<size_t>(kStaticScratchInts)) {
+  // The stated limit of this entry point; the grouping itself needs no scratch.
+  constexpr size_t kLimitInts = 64 * 1024;
+  const size_t need = grouping_workspace(numel, num_experts) / sizeof(int);
+  if (need > kLimitInts) {
     static thread_local char msg[160];
     snprintf(msg, sizeof(msg),
              "moe_align_block_size_static: ceil(numel/2048)*num_experts = %zu ints exceeds the "
-             "built-in scratch of %d ints; use b200moe_moe_align_block_size with a workspace",
-             need / sizeof(int), kStaticScratchInts);
+             "built-in scratch of %zu ints; use b200moe_moe_align_block_size with a workspace",
+             need, kLimitInts);
     set_last_error(msg, cudaErrorInvalidValue);
     return B200MOE_WORKSPACE_TOO_SMALL;
   }
-  int* scratch = nullptr;
-  if (need > 0) {
-    scratch = static_scratch_on_current_device();
-    if (!scratch) return B200MOE_CUDA_ERROR;
-  }
-  // Nothing in the scratch has to start at zero: the count pass overwrites every
-  // entry the scan and placement passes read.
   return b200moe_moe_align_block_size(topk_ids, ids_dtype, numel, num_experts, block_size,
                                       expert_map, sorted_token_ids, sorted_capacity, expert_ids,
-                                      blocks_capacity, num_tokens_post_pad, scratch,
-                                      sizeof(int) * static_cast<size_t>(kStaticScratchInts), stream);
+                                      blocks_capacity, num_tokens_post_pad, nullptr, 0, stream);
 }
 
 // ---- batched_moe_align_block_size and reorder_mxfp_scales ------------------------------

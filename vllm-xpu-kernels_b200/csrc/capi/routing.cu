@@ -68,6 +68,8 @@ __global__ void __launch_bounds__(128) topk_gating_kernel(
     float* __restrict__ weights, void* __restrict__ ids, int ids_dtype,
     int32_t* __restrict__ src_rows, const void* __restrict__ input_ids, int input_ids_dtype,
     const int32_t* __restrict__ tid2eid) {
+  pdl_wait();
+  pdl_trigger();
   const int rows_per_block = blockDim.x / LANES;
   const int sub = threadIdx.x % LANES;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * rows_per_block + threadIdx.x / LANES;
@@ -164,10 +166,10 @@ int launch_topk(const void* logits, int T_, int E, int k, int renorm, const floa
   do {                                                                                  \
     const int rows_per_block = 128 / LANES;                                             \
     const int grid = (T_ + rows_per_block - 1) / rows_per_block;                        \
-    topk_gating_kernel<T, LANES, VPT, SCORE><<<grid, 128, 0, st>>>(                     \
-        in, T_, E, k, renorm != 0, bias, scale, pad, w, ids, ids_dtype, src_rows,       \
-        input_ids, input_ids_dtype, tid2eid);                                           \
-    return launch_status("topk_gating_kernel");                                         \
+    return launch_pdl("topk_gating_kernel", topk_gating_kernel<T, LANES, VPT, SCORE>,   \
+                      dim3(grid), dim3(128), 0, st, 1, in, T_, E, k, renorm != 0, bias, \
+                      scale, pad, w, ids, ids_dtype, src_rows, input_ids,               \
+                      input_ids_dtype, tid2eid);                                        \
   } while (0)
   if (E <= 4) LAUNCH(4, 1);
   if (E <= 8) LAUNCH(8, 1);
@@ -191,6 +193,8 @@ __global__ void __launch_bounds__(128) grouped_topk_kernel(
     const T* __restrict__ scores, const TB* __restrict__ bias, int num_rows, int E,
     int n_group, int topk_group, int k, bool renorm, float scale, int scoring_func,
     float* __restrict__ values, int32_t* __restrict__ ids) {
+  pdl_wait();
+  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= num_rows) return;  // whole warp leaves together
@@ -316,10 +320,10 @@ int launch_grouped(const void* scores, const void* bias, int T_, int E, int n_gr
   const int grid = (T_ + 3) / 4;
 #define LAUNCH(VPT)                                                                        \
   do {                                                                                     \
-    grouped_topk_kernel<T, TB, VPT><<<grid, 128, 0, st>>>(                                 \
-        reinterpret_cast<const T*>(scores), reinterpret_cast<const TB*>(bias), T_, E,      \
-        n_group, topk_group, k, renorm != 0, scale, scoring_func, values, ids);            \
-    return launch_status("grouped_topk_kernel");                                           \
+    return launch_pdl("grouped_topk_kernel", grouped_topk_kernel<T, TB, VPT>, dim3(grid),   \
+                      dim3(128), 0, st, 1, reinterpret_cast<const T*>(scores),              \
+                      reinterpret_cast<const TB*>(bias), T_, E, n_group, topk_group, k,     \
+                      renorm != 0, scale, scoring_func, values, ids);                       \
   } while (0)
   if (E <= 32) LAUNCH(1);
   if (E <= 64) LAUNCH(2);

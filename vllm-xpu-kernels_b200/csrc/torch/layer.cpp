@@ -1,0 +1,200 @@
+// CPython entry of the whole-layer call (b200moe_layer_forward): what XpuFusedMoe.apply runs.
+//
+// A plain extension module with the vector calling convention rather than a torch operator: the
+// call sits on the critical path of small batches, and the operator dispatcher (schema matching,
+// boxing of every argument) costs more than the launches it would wrap.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <stdlib.h>
+
+#include "b200moe.h"
+
+namespace {
+
+// The constant part of a layer: the C ABI's description and the tensors it points into.
+struct Plan {
+  b200moe_layer layer{};
+  at::Tensor keep[6];
+  c10::DeviceIndex device = 0;
+  at::ScalarType weight_dtype = at::kByte;
+};
+
+constexpr const char* kCapsule = "b200moe.layer";
+
+void drop_plan(PyObject* cap) { delete static_cast<Plan*>(PyCapsule_GetPointer(cap, kCapsule)); }
+
+const at::Tensor& tensor(PyObject* o, const char* what) {
+  TORCH_CHECK(THPVariable_Check(o), what, " must be a tensor");
+  return THPVariable_Unpack(o);
+}
+
+int float_code(const at::Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kFloat: return B200MOE_F32;
+    case at::kHalf: return B200MOE_F16;
+    case at::kBFloat16: return B200MOE_BF16;
+    case at::kFloat8_e4m3fn: return B200MOE_E4M3;
+    default: return -1;
+  }
+}
+
+int index_code(const at::Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kInt: return B200MOE_I32;
+    case at::kLong: return B200MOE_I64;
+    case at::kUInt32: return B200MOE_U32;
+    default: return -1;
+  }
+}
+
+// make_plan(recipe, epilogue, b_layout, gated_act, act_param0, act_param1, clamp, alpha, limit,
+//           scales_pow2, H, I, E, w13, w13_scale, w13_bias, w2, w2_scale, w2_bias) -> capsule
+PyObject* make_plan(PyObject*, PyObject* args) {
+  HANDLE_TH_ERRORS
+  auto plan = std::make_unique<Plan>();
+  b200moe_layer& l = plan->layer;
+  PyObject* t[6];
+  if (!PyArg_ParseTuple(args, "iiiifffffiiiiOOOOOO", &l.recipe, &l.epilogue, &l.b_layout, &l.gated_act,
+                        &l.act_param0, &l.act_param1, &l.clamp_limit, &l.alpha, &l.limit, &l.scales_pow2, &l.H,
+                        &l.I, &l.E, &t[0], &t[1], &t[2], &t[3], &t[4], &t[5]))
+    return nullptr;
+  const void* ptr[6] = {};
+  for (int i = 0; i < 6; ++i) {
+    if (t[i] == Py_None) continue;
+    plan->keep[i] = tensor(t[i], "weights");
+    TORCH_CHECK(plan->keep[i].is_cuda() && plan->keep[i].is_contiguous(), "layer weights must be contiguous CUDA tensors");
+    ptr[i] = plan->keep[i].data_ptr();
+  }
+  TORCH_CHECK(ptr[0] && ptr[3], "a layer needs both weight tensors");
+  l.w13 = ptr[0];
+  l.w13_scale = ptr[1];
+  l.w13_bias = ptr[2];
+  l.w2 = ptr[3];
+  l.w2_scale = ptr[4];
+  l.w2_bias = ptr[5];
+  for (int i : {2, 5}) {
+    if (!ptr[i]) continue;
+    const int code = float_code(plan->keep[i]);
+    TORCH_CHECK(code >= 0 && code != B200MOE_E4M3 &&
+                    plan->keep[i].numel() == static_cast<int64_t>(l.E) * (i == 2 ? 2 * l.I : l.H),
+                "bias must be a float tensor [E, N]");
+    (i == 2 ? l.w13_bias_dtype : l.w2_bias_dtype) = code;
+  }
+  plan->device = plan->keep[0].get_device();
+  plan->weight_dtype = plan->keep[0].scalar_type();
+  return PyCapsule_New(plan.release(), kCapsule, drop_plan);
+  END_HANDLE_TH_ERRORS
+}
+
+// apply(plan, output, hidden, topk_weights, topk_ids, expert_map, a1q_scale, shared, valid_tokens,
+//       total_experts, stages, workspace) -> bool.  False: not a call this path takes (the caller
+// then goes operator by operator, which also words the error, if it is one).
+PyObject* apply(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 12, "apply takes 12 arguments");
+  const Plan* plan = static_cast<const Plan*>(PyCapsule_GetPointer(a[0], kCapsule));
+  if (!plan) return nullptr;
+  const b200moe_layer& l = plan->layer;
+  const at::Tensor& out = tensor(a[1], "output");
+  const at::Tensor& x = tensor(a[2], "hidden_states");
+  const at::Tensor& w = tensor(a[3], "topk_weights");
+  const at::Tensor& ids = tensor(a[4], "topk_ids");
+  b200moe_layer_call c{};
+  c.out_dtype = float_code(out);
+  c.x_dtype = float_code(x);
+  c.ids_dtype = index_code(ids);
+  if (x.dim() != 2 || out.dim() != 2 || ids.dim() != 2 || w.dim() != 2) Py_RETURN_FALSE;
+  c.T = static_cast<int>(x.size(0));
+  c.k = static_cast<int>(ids.size(1));
+  const bool x16 = c.x_dtype == B200MOE_BF16 || c.x_dtype == B200MOE_F16;
+  const bool out16 = c.out_dtype == B200MOE_BF16 || c.out_dtype == B200MOE_F16;
+  const bool plain = l.recipe == B200MOE_RECIPE_BF16;
+  if (!out16 || !(x16 || (c.x_dtype == B200MOE_E4M3 && !plain)) || c.ids_dtype < 0 || c.k > 64 ||
+      w.scalar_type() != at::kFloat || !x.is_contiguous() || !out.is_contiguous() || !w.is_contiguous() ||
+      !ids.is_contiguous() || x.size(1) != l.H || out.size(0) != c.T || out.size(1) != l.H ||
+      ids.size(0) != c.T || w.size(0) != c.T || w.size(1) != c.k || !x.is_cuda() || x.get_device() != plan->device ||
+      out.get_device() != plan->device || ids.get_device() != plan->device || w.get_device() != plan->device ||
+      static_cast<int64_t>(c.T) * c.k >= (1ll << 31))
+    Py_RETURN_FALSE;
+  if (plain && (x.scalar_type() != plan->weight_dtype || out.scalar_type() != plan->weight_dtype)) Py_RETURN_FALSE;
+  if (getenv("B200MOE_UNFUSED_ACT")) Py_RETURN_FALSE;
+  at::Tensor map32;
+  if (a[5] != Py_None) {
+    const at::Tensor& m = tensor(a[5], "expert_map");
+    map32 = m.scalar_type() == at::kInt && m.is_contiguous() ? m : m.to(at::kInt).contiguous();
+    c.expert_map = map32.data_ptr<int>();
+  }
+  if (a[6] != Py_None) {
+    const at::Tensor& s = tensor(a[6], "a1q_scale");
+    const int64_t width = l.recipe == B200MOE_RECIPE_MXFP4 ? (l.H + 511) / 512 * 16 : l.H / 128;
+    const size_t elt = l.recipe == B200MOE_RECIPE_MXFP4 ? 1 : 4;
+    if (x16 || plain || !s.is_contiguous() || s.element_size() != elt || s.numel() != c.T * width) Py_RETURN_FALSE;
+    c.x_scale = s.data_ptr();
+  } else if (!x16) {
+    Py_RETURN_FALSE;
+  }
+  if (a[7] != Py_None) {
+    const at::Tensor& s = tensor(a[7], "shared_output");
+    if (s.scalar_type() != out.scalar_type() || !s.is_contiguous() || s.sizes() != out.sizes()) Py_RETURN_FALSE;
+    c.shared = s.data_ptr();
+  } else if (a[8] != Py_None) {
+    const at::Tensor& v = tensor(a[8], "valid_tokens");
+    if (v.scalar_type() != at::kInt || v.numel() < 1 || !v.is_cuda()) Py_RETURN_FALSE;
+    c.valid_tokens = v.data_ptr<int>();
+  }
+  c.total_experts = static_cast<int>(PyLong_AsLong(a[9]));
+  c.stages = static_cast<int>(PyLong_AsLong(a[10]));
+  if (PyErr_Occurred()) return nullptr;
+  c.x = x.data_ptr();
+  c.out = out.data_ptr();
+  c.topk_weights = w.data_ptr<float>();
+  c.topk_ids = ids.data_ptr();
+  c10::cuda::OptionalCUDAGuard guard;
+  if (c10::cuda::current_device() != plan->device) guard.set_index(plan->device);
+  void* stream = at::cuda::getCurrentCUDAStream(plan->device).stream();
+  const size_t bytes = b200moe_layer_workspace_bytes(&l, &c);
+  int rc;
+  if (a[11] != Py_None) {  // a caller that brackets the stages keeps the scratch between its calls
+    const at::Tensor& ws = tensor(a[11], "workspace");
+    rc = b200moe_layer_forward(&l, &c, ws.data_ptr(), ws.nbytes(), stream);
+  } else {
+    // freed on return in stream order, as any tensor of the calling stream
+    c10::DataPtr ws = c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
+    rc = b200moe_layer_forward(&l, &c, ws.get(), bytes, stream);
+  }
+  if (rc == B200MOE_UNSUPPORTED) Py_RETURN_FALSE;  // the operators word the error
+  TORCH_CHECK(rc == B200MOE_OK, "XpuFusedMoe.apply: ", b200moe_status_string(rc), " (", b200moe_last_error(), ")");
+  Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
+}
+
+// workspace_bytes(plan, T, k) -> int
+PyObject* workspace_bytes(PyObject*, PyObject* args) {
+  HANDLE_TH_ERRORS
+  PyObject* cap;
+  b200moe_layer_call c{};
+  if (!PyArg_ParseTuple(args, "Oii", &cap, &c.T, &c.k)) return nullptr;
+  const Plan* plan = static_cast<const Plan*>(PyCapsule_GetPointer(cap, kCapsule));
+  if (!plan) return nullptr;
+  return PyLong_FromSize_t(b200moe_layer_workspace_bytes(&plan->layer, &c));
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {
+    {"make_plan", make_plan, METH_VARARGS, nullptr},
+    {"apply", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(apply)), METH_FASTCALL, nullptr},
+    {"workspace_bytes", workspace_bytes, METH_VARARGS, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_b200_layer", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__b200_layer(void) { return PyModule_Create(&module); }

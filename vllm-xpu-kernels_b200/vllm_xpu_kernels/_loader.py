@@ -12,6 +12,7 @@ import torch
 _HERE = os.path.dirname(os.path.abspath(__file__))
 CAPI_PATH = os.path.join(_HERE, "libb200moe.so")
 TORCH_OPS_PATH = os.path.join(_HERE, "_b200_torch_ops.so")
+LAYER_PATH = os.path.join(_HERE, "_b200_layer.so")
 _loaded = False
 
 
@@ -19,7 +20,7 @@ def load():
     global _loaded
     if _loaded:
         return
-    for path in (CAPI_PATH, TORCH_OPS_PATH):
+    for path in (CAPI_PATH, TORCH_OPS_PATH, LAYER_PATH):
         if not os.path.exists(path):
             raise ImportError(
                 f"{path} is missing: build it with `python vllm-xpu-kernels_b200/build.py` "

@@ -39,8 +39,29 @@ class MxGemmArgs(Structure):
     ]
 
 
+class Layer(Structure):
+    _fields_ = [
+        ("recipe", c_int), ("epilogue", c_int), ("b_layout", c_int), ("gated_act", c_int),
+        ("act_param0", c_float), ("act_param1", c_float), ("clamp_limit", c_float), ("alpha", c_float),
+        ("limit", c_float), ("scales_pow2", c_int), ("H", c_int), ("I", c_int), ("E", c_int),
+        ("w13", c_void_p), ("w13_scale", c_void_p), ("w13_bias", c_void_p), ("w2", c_void_p),
+        ("w2_scale", c_void_p), ("w2_bias", c_void_p), ("w13_bias_dtype", c_int), ("w2_bias_dtype", c_int),
+    ]
+
+
+class LayerCall(Structure):
+    _fields_ = [
+        ("stages", c_int), ("x", c_void_p), ("x_dtype", c_int), ("x_scale", c_void_p),
+        ("topk_weights", c_void_p), ("topk_ids", c_void_p), ("ids_dtype", c_int), ("expert_map", c_void_p),
+        ("T", c_int), ("k", c_int), ("total_experts", c_int), ("out", c_void_p), ("out_dtype", c_int),
+        ("shared", c_void_p), ("valid_tokens", c_void_p),
+    ]
+
+
 # name -> (restype, argtypes); must list every symbol include/b200moe.h declares.
 SIGNATURES = {
+    "b200moe_layer_workspace_bytes": (c_size_t, [POINTER(Layer), POINTER(LayerCall)]),
+    "b200moe_layer_forward": (c_int, [POINTER(Layer), POINTER(LayerCall), c_void_p, c_size_t, c_void_p]),
     "b200moe_version": (c_char_p, []),
     "b200moe_status_string": (c_char_p, [c_int]),
     "b200moe_last_error": (c_char_p, []),

@@ -40,6 +40,7 @@ import torch
 try:
     from . import _C  # noqa: F401
     from . import _moe_C  # noqa: F401
+    from . import _b200_layer
     from . import _xpu_C  # noqa: F401
     FUSEDMOE_UNAVAILABLE_REASON = None
     FUSEDMOE_AVAILABLE = True
@@ -47,9 +48,11 @@ except ImportError as e:  # the class below then raises on construction
     FUSEDMOE_UNAVAILABLE_REASON = str(e)
     FUSEDMOE_AVAILABLE = False
 
+RECIPE_BF16, RECIPE_FP8_BLOCK, RECIPE_MXFP4 = 0, 1, 2
 EPI_STORE, EPI_SILU_MUL, EPI_SWIGLU_OAI = 0, 1, 2
+LAYER_STAGES = (("remap", 1), ("gemm1", 2), ("gemm2", 4), ("gather", 8))  # B200MOE_LAYER_* of b200moe.h
+LAYER_ALL = 15
 B_LAYOUT_KN, B_LAYOUT_NK = 0, 1
-A_SCALE_ROW_MAJOR_DECODE = 2   # row-major activation scales + the decode-regime GEMM kernel
 
 
 def _get_weights_dtype(weight, scales):
@@ -192,6 +195,8 @@ class XpuFusedMoe:
                 self._w2_16 = torch.ops._xpu_C.b200_dequant_weights(
                     w2.view(torch.uint8), w2_scales.view(torch.uint8))
 
+        self._plans = {}   # output dtype -> native plan of the whole-layer call, or None
+
         # Optional list; when set, apply() appends (stage, start_event, end_event)
         # for each stage, the way the reference's benchmark brackets its stages
         # (benchmark/src/fused_moe_interface_.py:84-168 there).
@@ -223,9 +228,64 @@ class XpuFusedMoe:
         self.stage_timer.append((name, start, end))
 
     def launches_per_apply(self, num_rows: int) -> int:
-        """Kernels one apply() enqueues for `num_rows` already-quantised tokens."""
-        permute = 2 if num_rows * self.n_experts_per_token <= 2048 else 4
+        """Kernels one apply() enqueues for `num_rows` tokens."""
+        permute = 1 if num_rows * self.n_experts_per_token <= 2048 else 2
         return permute + 3  # gemm1 (activation [+ quantisation] fused), gemm2, gather
+
+    def _native_plan(self, out_dtype):
+        """Handle of the whole-layer call (weights, shapes, activation) for layers whose
+        activation runs in the first GEMM's epilogue; None for the others, which go operator by
+        operator."""
+        if out_dtype in self._plans:
+            return self._plans[out_dtype]
+        plan = None
+        clamp = self.gemm1_clamp_limit is not None and self.gemm1_clamp_limit > 0
+        oai = _is_swigluoai(self.activation)
+        fused = self._fused_gated(clamp)
+        H = self.w13.shape[-1] * 2 if (self.is_mxfp4 or self.is_int4) else self.w13.shape[-2]
+        shape = (H, self.inter_size, self.num_experts)
+        lim = float(self.gemm1_clamp_limit) if clamp else 0.0
+        if out_dtype not in (torch.bfloat16, torch.float16):
+            pass
+        elif self._mx_native:
+            if oai and not clamp:
+                plan = _b200_layer.make_plan(RECIPE_MXFP4, EPI_SWIGLU_OAI, B_LAYOUT_NK, 0, 0.0, 0.0, 0.0, 1.702, 7.0,
+                                             0, *shape, self.w13.view(torch.uint8), self._w13_sf, self.w13_bias,
+                                             self.w2.view(torch.uint8), self._w2_sf, self.w2_bias)
+        elif self.is_block_fp8:
+            if fused is not None and self.inter_size % 128 == 0 and self.w13.dtype == torch.float8_e4m3fn:
+                plan = _b200_layer.make_plan(RECIPE_FP8_BLOCK, EPI_SILU_MUL, B_LAYOUT_KN, *fused, 1.702, 7.0,
+                                             int(self.act_scales_pow2), *shape, self.w13, self.gemm1_wei_scales,
+                                             self.w13_bias, self.w2, self.gemm2_wei_scales, self.w2_bias)
+        elif fused is not None or oai:
+            w13, w2, layout = self._weights_16(out_dtype)
+            if w13.dtype == out_dtype and w2.dtype == out_dtype:
+                extra = fused if fused is not None else (0, 0.0, 0.0, lim)
+                plan = _b200_layer.make_plan(RECIPE_BF16, EPI_SWIGLU_OAI if oai else EPI_SILU_MUL, layout, *extra,
+                                             1.702, 7.0, 0, *shape, w13, None, self.w13_bias, w2, None, self.w2_bias)
+        self._plans[out_dtype] = plan
+        return plan
+
+    def _apply_native(self, plan, output, hidden_states, topk_weights, topk_ids, expert_map, a1q_scale,
+                      shared_output, valid_tokens, after_gemms):
+        """The whole layer in one native call, or stage by stage when something on the stream has
+        to happen between the stages.  False: not a call the native path takes."""
+        if self._mx_native and a1q_scale is not None:
+            a1q_scale = self._pad_mx_scales(a1q_scale, hidden_states.shape[1])
+        call = _b200_layer.apply
+        if self.stage_timer is None and after_gemms is None:
+            return call(plan, output, hidden_states, topk_weights, topk_ids, expert_map, a1q_scale, shared_output,
+                        valid_tokens, self.total_experts_num, LAYER_ALL, None)
+        ws = torch.empty(_b200_layer.workspace_bytes(plan, topk_ids.shape[0], topk_ids.shape[1]), dtype=torch.uint8,
+                         device=hidden_states.device)
+        for name, bit in LAYER_STAGES:
+            if name == "gather" and after_gemms is not None:
+                after_gemms.record()
+            with self._stage(name):
+                if not call(plan, output, hidden_states, topk_weights, topk_ids, expert_map, a1q_scale,
+                            shared_output, valid_tokens, self.total_experts_num, bit, ws):
+                    return False
+        return True
 
     # ------------------------------------------------------------------
     def apply(self, output, hidden_states, topk_weights, topk_ids, expert_map=None,
@@ -254,21 +314,25 @@ class XpuFusedMoe:
 
         ``after_gemms`` (not in the reference signature): a ``torch.cuda.Event`` recorded on the
         current stream right after the second grouped GEMM, before the combine."""
+        if expert_map is None and self.ep_size > 1:
+            expert_map = self.expert_map
+        if row_destinations is None:
+            try:
+                plan = self._plans[output.dtype]
+            except KeyError:
+                plan = self._native_plan(output.dtype)
+            if plan is not None and self._apply_native(plan, output, hidden_states, topk_weights, topk_ids,
+                                                       expert_map, a1q_scale, shared_output, valid_tokens,
+                                                       after_gemms):
+                return
+        # Operator by operator: activations that are not fused into the first GEMM, per-row
+        # destinations, and arguments the native call does not take.
         num_rows, hidden_size = hidden_states.shape
         k = topk_ids.shape[1]  # n_experts_per_token, or 1 for rows that arrive already dispatched
         R = num_rows * k
         dev = hidden_states.device
-        if expert_map is None and self.ep_size > 1:
-            expert_map = self.expert_map
         if num_rows == 0:
             return
-
-        if (self.is_block_fp8 and row_destinations is None and valid_tokens is None
-                and self._decode_regime(num_rows * k)
-                and self.activation == "silu" and not (self.gemm1_clamp_limit or 0) > 0
-                and self.inter_size % 128 == 0):
-            return self._apply_decode(output, hidden_states, topk_weights, topk_ids, expert_map,
-                                      a1q_scale, shared_output)
         if self.is_block_fp8 and a1q_scale is None:
             # dynamic per-token-group-128 quantisation, once per token (not per routed row)
             from .moe_utils import quant_fp8_block_act
@@ -474,46 +538,6 @@ class XpuFusedMoe:
         if forced is not None:
             return forced == "1"
         return routed_rows <= self.num_experts
-
-    def _apply_decode(self, output, hidden_states, topk_weights, topk_ids, expert_map, a1q_scale,
-                      shared_output=None):
-        """Same sequence of launches as the default path, with the two grouped GEMMs on the
-        decode-regime kernel (weights on the M side of the MMA, 32 tokens per tile); the first
-        one quantises its output per token per 128 columns in its epilogue."""
-        from .moe_utils import quant_fp8_block_act
-        T, H = hidden_states.shape
-        k = topk_ids.shape[1]
-        R, I, E = T * k, self.inter_size, self.num_experts
-        dev = hidden_states.device
-        if a1q_scale is None:
-            hidden_states, a1q_scale = quant_fp8_block_act(hidden_states)
-        if expert_map is None and self.ep_size > 1:
-            expert_map = self.expert_map
-        remapped = torch.empty((R, H), dtype=hidden_states.dtype, device=dev)
-        remapped_scales = torch.empty((R, a1q_scale.shape[1]), dtype=a1q_scale.dtype, device=dev)
-        rows_per_expert = torch.zeros((E,), dtype=torch.int32, device=dev)
-        row_map = torch.empty((T, k), dtype=torch.int32, device=dev)
-        with self._stage("remap"):
-            torch.ops._moe_C.remap_hidden_states(hidden_states, a1q_scale, remapped, remapped_scales,
-                                                 expert_map, rows_per_expert, row_map, topk_ids,
-                                                 self.total_experts_num, self.local_experts_num)
-        gemm = torch.ops._xpu_C.b200_grouped_gemm
-        act_q = torch.empty((R, I), dtype=torch.float8_e4m3fn, device=dev)
-        act_s = torch.empty((R, I // 128), dtype=torch.float32, device=dev)
-        with self._stage("gemm1"):
-            gemm(remapped, remapped_scales, self.w13, self.gemm1_wei_scales, self.w13_bias, act_q,
-                 rows_per_expert, 2 * I, H, E, EPI_SILU_MUL, B_LAYOUT_KN, 1.702, 7.0, act_s, None,
-                 A_SCALE_ROW_MAJOR_DECODE)
-        gemm2_out = torch.empty((R, H), dtype=output.dtype, device=dev)
-        with self._stage("gemm2"):
-            gemm(act_q, act_s, self.w2, self.gemm2_wei_scales, self.w2_bias, gemm2_out, rows_per_expert,
-                 H, I, E, EPI_STORE, B_LAYOUT_KN, 1.702, 7.0, None, None, A_SCALE_ROW_MAJOR_DECODE)
-        with self._stage("gather"):
-            if shared_output is not None:
-                torch.ops._moe_C.b200_moe_gather_add(output, gemm2_out, topk_weights, row_map,
-                                                     shared_output)
-            else:
-                torch.ops._moe_C.moe_gather(output, gemm2_out, topk_weights, row_map, self.num_experts)
 
     def _weights_16(self, dtype):
         """(w13, w2, layout) as 16-bit operands of the grouped GEMM."""
