@@ -671,7 +671,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     prefetch_tensormap(&map_b);
   }
   pdl_wait();   // everything below reads what earlier kernels wrote
-  pdl_trigger();
   build_schedule(sched, p.rows_per_expert, p.E, p.R, n_tiles, C::TILE_M);
   if (warp == 1) {
     if constexpr (C::PAIR) {
@@ -1102,6 +1101,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     }
   }
 
+  pdl_trigger();
   // ---------------- teardown ----------------
   tc_fence_before();
   __syncthreads();
@@ -1222,7 +1222,7 @@ int launch_config(const b200moe_gemm_args& a, const void* B, int b_dtype, cudaSt
   if (grid < 1) grid = 1;
   if (C::PAIR) grid = grid < 2 ? 2 : grid & ~1ll;
   return launch_pdl("grouped_gemm_kernel", grouped_gemm_kernel<C>, dim3(static_cast<unsigned>(grid)),
-                    dim3(C::THREADS), C::SMEM_BYTES, st, C::PAIR ? 2 : 1, map_a, map_b, p);
+                    dim3(C::THREADS), C::SMEM_BYTES, st, C::PAIR ? 2 : 1, a.R, map_a, map_b, p);
 }
 
 // ---- CUDA-core evaluation of the same contract (checking aid) --------------------------

@@ -186,7 +186,6 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_tok,
     prefetch_tensormap(&map_w);
   }
   pdl_wait();
-  pdl_trigger();
   build_decode_schedule(sched, p.rows_per_expert, p.E, p.R, f_tiles);
   if (warp == 1) {
     tmem_alloc(&tmem_base_slot, C::TMEM_COLS);
@@ -405,6 +404,7 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_tok,
     }
   }
 
+  pdl_trigger();
   tc_fence_before();
   __syncthreads();
   if (abort_flag) {
@@ -449,7 +449,7 @@ int launch_decode(const b200moe_gemm_args& a, cudaStream_t st) {
       decode_gemm_kernel<GATED>, C::SMEM_BYTES + kMaxDecodeKBlocks * (kNTok + 2) * sizeof(float),
       "cudaFuncSetAttribute");
   if (arc != B200MOE_OK) return arc;
-  return launch_pdl("decode_gemm_kernel", decode_gemm_kernel<GATED>, dim3(kNumSMs), dim3(C::THREADS), smem, st, 1,
+  return launch_pdl("decode_gemm_kernel", decode_gemm_kernel<GATED>, dim3(kNumSMs), dim3(C::THREADS), smem, st, 1, a.R,
                     map_tok, map_w, p);
 }
 

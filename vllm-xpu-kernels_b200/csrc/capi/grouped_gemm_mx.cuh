@@ -186,7 +186,6 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
     prefetch_tensormap(&map_b_tail);
   }
   pdl_wait();
-  pdl_trigger();
   build_schedule(sched, p.rows_per_expert, p.E, p.R, n_tiles, BM);
   if (warp == 1) {
     tmem_alloc(&tmem_base_slot, C::TMEM_COLS);
@@ -402,6 +401,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
     }
   }
 
+  pdl_trigger();
   // ---------------- teardown ----------------
   tc_fence_before();
   __syncthreads();
@@ -477,7 +477,7 @@ int launch_mx(const b200moe_mx_gemm_args& a, cudaStream_t st) {
   if (grid > kNumSMs) grid = kNumSMs;
   if (grid < 1) grid = 1;
   return launch_pdl("grouped_gemm_mx_kernel", grouped_gemm_mx_kernel<C>, dim3(static_cast<unsigned>(grid)),
-                    dim3(C::THREADS), C::SMEM_BYTES, st, 1, map_a, map_b, map_b_tail, p);
+                    dim3(C::THREADS), C::SMEM_BYTES, st, 1, a.R, map_a, map_b, map_b_tail, p);
 }
 
 // Weight scales [E, N, K/32] (e8m0 bytes) -> [E, ceil(K/128), ceil(N/128)+1, 512]: per

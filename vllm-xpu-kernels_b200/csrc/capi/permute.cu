@@ -411,13 +411,13 @@ int run_grouping(const GroupParams& p, const AlignOut& ao, int32_t* rows_per_key
   if (p.num_keys > kMaxExperts) return B200MOE_UNSUPPORTED;
   if (p.numel <= kChunk)
     return launch_pdl("fused_small_kernel", fused_small_kernel, dim3(1), dim3(kThreads),
-                      p.num_keys * kWarps * sizeof(int), st, 1, p, ao, rows_per_key, accumulate, row_map);
+                      p.num_keys * kWarps * sizeof(int), st, 1, p.numel, p, ao, rows_per_key, accumulate, row_map);
   struct Tag {};
   const int rc = ensure_dynamic_smem<Tag>(group_cluster_kernel, kMaxExperts * kGroupWarps * sizeof(int),
                                           "cudaFuncSetAttribute (grouping)");
   if (rc != B200MOE_OK) return rc;
   return launch_pdl("group_cluster_kernel", group_cluster_kernel, dim3(kGroupCtas), dim3(kGroupThreads),
-                    static_cast<size_t>(p.num_keys) * kGroupWarps * sizeof(int), st, 1, p, ao, rows_per_key,
+                    static_cast<size_t>(p.num_keys) * kGroupWarps * sizeof(int), st, 1, p.numel, p, ao, rows_per_key,
                     accumulate, row_map);
 }
 
@@ -609,7 +609,7 @@ int permute_rows(const PermuteRows& a, cudaStream_t st) {
   if (parts < 1) parts = 1;
   const dim3 grid(a.T, parts);
   auto go = [&](auto kernel) {
-    return launch_pdl("rows_kernel", kernel, grid, dim3(kThreads), 0, st, 1, g, p);
+    return launch_pdl("rows_kernel", kernel, grid, dim3(kThreads), 0, st, 1, g.numel, g, p);
   };
   const bool f16 = a.src_dtype == B200MOE_F16;
   if (a.mode == ROW_QUANT_FP8) {

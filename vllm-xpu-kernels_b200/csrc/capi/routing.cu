@@ -1,10 +1,13 @@
 // Routing kernels: softmax / sigmoid top-k and DeepSeek grouped top-k.
 //
 // All three are warp-level: a row's scores live in registers (expert
-// e = lane + LANES*i), the k winners are found by k rounds of a butterfly
-// arg-max whose order is (key descending, expert index ascending) — the order
-// a stable descending sort gives — and nothing touches shared memory or a
-// workspace.  Scores are computed with IEEE division and the accurate expf so
+// e = lane + LANES*i), the k winners are found by k rounds of an arg-max whose
+// order is (key descending, expert index ascending) — the order a stable
+// descending sort gives — and nothing touches shared memory or a workspace.
+// A round is a chain of dependent steps, and k rounds of it are the kernel (a
+// few bytes per row): for whole-warp rows the arg-max is two warp reductions on
+// integers that sort like the keys instead of five exchange steps of three
+// shuffles each.  Measured, 256 experts, 8 groups, top-8: see grouped_topk_kernel.  Scores are computed with IEEE division and the accurate expf so
 // that they agree with a plain fp32 evaluation of the same formula.
 #include <math_constants.h>
 
@@ -55,6 +58,46 @@ __device__ __forceinline__ float group_sum(float v) {
 }
 
 constexpr int kInvalidIdx = 0x7fffffff;
+
+// Unsigned integer that sorts like the float (+0 and -0 equal); 0 = not selectable, which is
+// what a NaN is too (it compares greater than nothing).
+__device__ __forceinline__ uint32_t sortable(float key) {
+  const uint32_t b = __float_as_uint(key + 0.0f);
+  return key != key ? 0u : (b & 0x80000000u ? ~b : b | 0x80000000u);
+}
+
+__device__ __forceinline__ float from_sortable(uint32_t u) {
+  if (u == 0u) return -CUDART_INF_F;
+  return __uint_as_float(u & 0x80000000u ? u & 0x7FFFFFFFu : ~u);
+}
+
+// Index (lane + 32 * i) of the largest of the warp's 32 * VPT keys, the lowest index among
+// equals; kInvalidIdx when nothing is selectable.  The winner's key is cleared.
+template <int VPT>
+__device__ __forceinline__ int take_best(uint32_t (&u)[VPT], int lane) {
+  uint32_t bu = u[0];
+  int bi = 0;
+#pragma unroll
+  for (int i = 1; i < VPT; ++i)
+    if (u[i] > bu) { bu = u[i]; bi = i; }
+  const uint32_t top = __reduce_max_sync(0xffffffffu, bu);
+  if (top == 0u) return kInvalidIdx;
+  const int idx = __reduce_min_sync(0xffffffffu, bu == top ? lane + 32 * bi : kInvalidIdx);
+#pragma unroll
+  for (int i = 0; i < VPT; ++i)
+    if (idx == lane + 32 * i) u[i] = 0u;
+  return idx;
+}
+
+// Value of array element idx = lane + 32 * i, from the lane that holds it to all.
+template <int VPT>
+__device__ __forceinline__ float value_at(const float (&s)[VPT], int idx) {
+  float v = 0.f;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i)
+    if ((idx >> 5) == i) v = s[i];
+  return __shfl_sync(0xffffffffu, v, idx & 31);
+}
 
 enum : int { SCORE_SOFTMAX = 0, SCORE_SIGMOID = 1, SCORE_SOFTPLUS_SQRT = 2 };
 
@@ -116,10 +159,20 @@ __global__ void __launch_bounds__(128) topk_gating_kernel(
   int my_id = 0;
   float wsum = 0.f;
   const int64_t hash_row = tid2eid ? load_index(input_ids, input_ids_dtype, r) * k : 0;
+  uint32_t sort_key[LANES == 32 ? VPT : 1];
+  if constexpr (LANES == 32) {
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) sort_key[i] = sub + 32 * i < E ? sortable(key[i]) : 0u;
+  }
   for (int j = 0; j < k; ++j) {
     Best b{-CUDART_INF_F, kInvalidIdx};
     float pay = 0.f;
-    if (tid2eid) {
+    if (LANES == 32 && !tid2eid) {
+      if constexpr (LANES == 32) {
+        b.idx = take_best<VPT>(sort_key, sub);
+        if (b.idx != kInvalidIdx) pay = value_at<VPT>(s, b.idx);
+      }
+    } else if (tid2eid) {
       b.idx = tid2eid[hash_row + j];
 #pragma unroll
       for (int i = 0; i < VPT; ++i)
@@ -167,7 +220,8 @@ int launch_topk(const void* logits, int T_, int E, int k, int renorm, const floa
     const int rows_per_block = 128 / LANES;                                             \
     const int grid = (T_ + rows_per_block - 1) / rows_per_block;                        \
     return launch_pdl("topk_gating_kernel", topk_gating_kernel<T, LANES, VPT, SCORE>,   \
-                      dim3(grid), dim3(128), 0, st, 1, in, T_, E, k, renorm != 0, bias, \
+                      dim3(grid), dim3(128), 0, st, 1, static_cast<int64_t>(T_) * k,    \
+                      in, T_, E, k, renorm != 0, bias,                                  \
                       scale, pad, w, ids, ids_dtype, src_rows, input_ids,               \
                       input_ids_dtype, tid2eid);                                        \
   } while (0)
@@ -224,44 +278,57 @@ __global__ void __launch_bounds__(128) grouped_topk_kernel(
   // Group score = sum of the two largest keys in the group; lane g ends up
   // holding group g's score.
   float my_group_score = -CUDART_INF_F;
-  for (int g = 0; g < n_group; ++g) {
-    const int lo = g * per, hi = lo + per;
-    float m1 = -CUDART_INF_F, m2 = -CUDART_INF_F;
+  if (per == 32) {
+    // group g is register g of every lane: the two largest by warp reductions
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int e = lane + 32 * i;
-      if (e >= lo && e < hi) {
-        const float v = key[i];
-        if (v > m1) { m2 = m1; m1 = v; } else if (v > m2) { m2 = v; }
+    for (int g = 0; g < VPT; ++g) {
+      if (g >= n_group) break;
+      const uint32_t u = sortable(key[g]);
+      const uint32_t t1 = __reduce_max_sync(0xffffffffu, u);
+      const uint32_t at = __ballot_sync(0xffffffffu, u == t1);
+      const uint32_t rest = __reduce_max_sync(0xffffffffu, u == t1 ? 0u : u);
+      const uint32_t t2 = (at & (at - 1)) ? t1 : rest;
+      float gs = from_sortable(t1) + from_sortable(t2);
+      if (kSameHalfType) gs = round_through<T>(gs);
+      if (lane == g) my_group_score = gs;
+    }
+  } else {
+    for (int g = 0; g < n_group; ++g) {
+      const int lo = g * per, hi = lo + per;
+      float m1 = -CUDART_INF_F, m2 = -CUDART_INF_F;
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        const int e = lane + 32 * i;
+        if (e >= lo && e < hi) {
+          const float v = key[i];
+          if (v > m1) { m2 = m1; m1 = v; } else if (v > m2) { m2 = v; }
+        }
       }
-    }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const float o1 = __shfl_xor_sync(0xffffffffu, m1, off);
-      const float o2 = __shfl_xor_sync(0xffffffffu, m2, off);
-      const float n1 = fmaxf(m1, o1);
-      const float n2 = fmaxf(fminf(m1, o1), fmaxf(m2, o2));
-      m1 = n1;
-      m2 = n2;
+      for (int off = 16; off > 0; off >>= 1) {
+        const float o1 = __shfl_xor_sync(0xffffffffu, m1, off);
+        const float o2 = __shfl_xor_sync(0xffffffffu, m2, off);
+        const float n1 = fmaxf(m1, o1);
+        const float n2 = fmaxf(fminf(m1, o1), fmaxf(m2, o2));
+        m1 = n1;
+        m2 = n2;
+      }
+      float gs = m1 + m2;
+      if (kSameHalfType) gs = round_through<T>(gs);
+      if (lane == g) my_group_score = gs;
     }
-    float gs = m1 + m2;
-    if (kSameHalfType) gs = round_through<T>(gs);
-    if (lane == g) my_group_score = gs;
   }
 
   // Stable top-`topk_group` over the n_group (<= 32) group scores.
   uint32_t group_mask = 0;
   float last_group_score = -CUDART_INF_F;
   {
-    bool taken = lane >= n_group;
+    uint32_t u[1] = {lane < n_group ? sortable(my_group_score) : 0u};
     for (int j = 0; j < topk_group; ++j) {
-      Best b{taken ? -CUDART_INF_F : my_group_score, taken ? kInvalidIdx : lane};
-      float pay = 0.f;
-      b = group_argmax<32>(b, pay);
-      last_group_score = b.idx == kInvalidIdx ? -CUDART_INF_F : b.key;
-      if (b.idx == kInvalidIdx) break;
-      group_mask |= 1u << b.idx;
-      if (b.idx == lane) taken = true;
+      const int best = take_best<1>(u, lane);
+      last_group_score = best == kInvalidIdx ? -CUDART_INF_F : __shfl_sync(0xffffffffu, my_group_score, best & 31);
+      if (best == kInvalidIdx) break;
+      group_mask |= 1u << best;
     }
   }
   // Fewer than `topk_group` groups with a finite score: the reference kernel gives up on the
@@ -279,28 +346,19 @@ __global__ void __launch_bounds__(128) grouped_topk_kernel(
     if (e < E && (!((group_mask >> (e / per)) & 1u) || ((inf_in >> i) & 1u))) key[i] = -CUDART_INF_F;
   }
 
-  uint32_t taken = 0;
+  uint32_t u[VPT];
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) u[i] = lane + 32 * i < E ? sortable(key[i]) : 0u;
   float my_w = 0.f;
   int my_id = 0;
   float wsum = 0.f;
   for (int j = 0; j < k; ++j) {
-    Best b{-CUDART_INF_F, kInvalidIdx};
-    float pay = 0.f;
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int e = lane + 32 * i;
-      if (e < E && !((taken >> i) & 1u) && better(key[i], e, b.key, b.idx)) {
-        b.key = key[i];
-        b.idx = e;
-        pay = s[i];
-      }
-    }
-    b = group_argmax<32>(b, pay);
-    if (b.idx != kInvalidIdx && (b.idx & 31) == lane) taken |= 1u << (b.idx >> 5);
+    const int best = take_best<VPT>(u, lane);
+    const float pay = best == kInvalidIdx ? 0.f : value_at<VPT>(s, best);
     wsum += pay;
     if (j == lane) {
       my_w = pay;
-      my_id = b.idx == kInvalidIdx ? 0 : b.idx;
+      my_id = best == kInvalidIdx ? 0 : best;
     }
   }
   if (lane < k) {
@@ -321,7 +379,8 @@ int launch_grouped(const void* scores, const void* bias, int T_, int E, int n_gr
 #define LAUNCH(VPT)                                                                        \
   do {                                                                                     \
     return launch_pdl("grouped_topk_kernel", grouped_topk_kernel<T, TB, VPT>, dim3(grid),   \
-                      dim3(128), 0, st, 1, reinterpret_cast<const T*>(scores),              \
+                      dim3(128), 0, st, 1, static_cast<int64_t>(T_) * k,                    \
+                      reinterpret_cast<const T*>(scores),                                   \
                       reinterpret_cast<const TB*>(bias), T_, E, n_group, topk_group, k,     \
                       renorm != 0, scale, scoring_func, values, ids);                       \
   } while (0)
