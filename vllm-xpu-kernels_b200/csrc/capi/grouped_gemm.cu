@@ -598,14 +598,25 @@ __device__ __forceinline__ void tile_epilogue(const GemmParams& p, const TileCoo
   }
 }
 
+// Rows of A a tile loads per stage.  A tile with few rows (experts of a small batch, ragged
+// ends) does not pull the 128 rows the MMA reads: boxes of kSmallBox rows up to the last valid
+// one are loaded and the rest of the stage keeps whatever it held -- accumulator rows are
+// independent and rows past the expert's end are never stored.  With one row per expert the
+// 128-row boxes were half of all bytes into the SMs (16 KB beside 16 KB of weights per stage).
+constexpr int kSmallBox = 32;
+__device__ __forceinline__ int small_boxes(int rows_valid) {
+  return rows_valid > BM - kSmallBox ? 0 : (rows_valid + kSmallBox - 1) / kSmallBox;   // 0: one whole box
+}
+
 // One pipeline stage of operands for K block `kb` of tile `tc`: this CTA's A box
 // (its 128 rows) and its B box(es).  In a CTA pair, rank 1 takes the second 128 rows
 // and the second half of the tile's columns, and every load reports to the leader's
 // barrier.
 template <typename C>
-__device__ __forceinline__ void issue_stage(const CUtensorMap& map_a, const CUtensorMap& map_b,
-                                            const GemmParams& p, const TileCoord& tc, int kb,
-                                            int rank, uint8_t* stage_smem, uint64_t* bar) {
+__device__ __forceinline__ void issue_stage(const CUtensorMap& map_a, const CUtensorMap& map_a_small,
+                                            const CUtensorMap& map_b, const GemmParams& p,
+                                            const TileCoord& tc, int small, int kb, int rank,
+                                            uint8_t* stage_smem, uint64_t* bar) {
   uint8_t* a_dst = stage_smem;
   uint8_t* b_dst = stage_smem + C::A_BYTES;
   auto b_box = [&](int off, int x, int y, int z) {
@@ -613,7 +624,11 @@ __device__ __forceinline__ void issue_stage(const CUtensorMap& map_a, const CUte
     else tma_load_3d(b_dst + off, &map_b, bar, x, y, z);
   };
   if constexpr (C::PAIR) tma_load_2d_pair(a_dst, &map_a, bar, kb * C::BK, tc.row_start + rank * BM);
-  else tma_load_2d(a_dst, &map_a, bar, kb * C::BK, tc.row_start);
+  else if (!small) tma_load_2d(a_dst, &map_a, bar, kb * C::BK, tc.row_start);
+  else
+    for (int i = 0; i < small; ++i)
+      tma_load_2d(a_dst + i * (kSmallBox * kStageRowBytes), &map_a_small, bar, kb * C::BK,
+                  tc.row_start + i * kSmallBox);
   const int tcol0 = rank * C::B_COLS;  // first tile column this CTA loads
   if constexpr (C::B_MN_MAJOR) {
 #pragma unroll
@@ -631,6 +646,7 @@ __device__ __forceinline__ void issue_stage(const CUtensorMap& map_a, const CUte
 template <typename C>
 __global__ void __launch_bounds__(C::THREADS, 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
+                    const __grid_constant__ CUtensorMap map_a_small,
                     const __grid_constant__ CUtensorMap map_b, GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ Schedule sched;
@@ -668,6 +684,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     }
     mbar_fence_init();
     prefetch_tensormap(&map_a);
+    if constexpr (!C::PAIR) prefetch_tensormap(&map_a_small);
     prefetch_tensormap(&map_b);
   }
   pdl_wait();   // everything below reads what earlier kernels wrote
@@ -701,14 +718,16 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       bool ok = true;
       for (int t = sched_id; t < num_tiles && ok; t += sched_stride) {
         const TileCoord tc = decode_tile(sched, t);
+        const int small = C::PAIR ? 0 : small_boxes(tc.rows_valid);
+        const uint32_t stage_tx = small ? small * (kSmallBox * kStageRowBytes) + C::B_BYTES
+                                        : C::STAGE_BYTES * (C::PAIR ? 2 : 1);
         for (int kb = 0; kb < num_kb && ok; ++kb) {
           ok = mbar_wait_warp(&bars.empty[stage], phase ^ 1u, abort_p);
           if (!ok) break;
           if (elect_one()) {
             // the leader's barrier counts the bytes of both CTAs of a pair
-            if (rank == 0)
-              mbar_arrive_expect_tx(&bars.full[stage], C::STAGE_BYTES * (C::PAIR ? 2 : 1));
-            issue_stage<C>(map_a, map_b, p, tc, kb, rank, tiles + stage * C::STAGE_BYTES,
+            if (rank == 0) mbar_arrive_expect_tx(&bars.full[stage], stage_tx);
+            issue_stage<C>(map_a, map_a_small, map_b, p, tc, small, kb, rank, tiles + stage * C::STAGE_BYTES,
                            &bars.full[stage]);
           }
           __syncwarp();
@@ -1172,8 +1191,9 @@ int make_map(CUtensorMap* map, int dtype, const void* base, uint64_t cols, uint6
 
 template <typename C>
 int launch_config(const b200moe_gemm_args& a, const void* B, int b_dtype, cudaStream_t st) {
-  CUtensorMap map_a, map_b;
+  CUtensorMap map_a, map_a_small, map_b;
   int rc = make_map(&map_a, a.a_dtype, a.A, a.K, a.R, 0, C::BK, BM);
+  if (rc == B200MOE_OK) rc = make_map(&map_a_small, a.a_dtype, a.A, a.K, a.R, 0, C::BK, kSmallBox);
   if (rc != B200MOE_OK) return rc;
   if (C::B_MN_MAJOR)
     rc = make_map(&map_b, b_dtype, B, a.N, a.K, a.E, C::CHUNK_COLS, C::BK);
@@ -1222,7 +1242,8 @@ int launch_config(const b200moe_gemm_args& a, const void* B, int b_dtype, cudaSt
   if (grid < 1) grid = 1;
   if (C::PAIR) grid = grid < 2 ? 2 : grid & ~1ll;
   return launch_pdl("grouped_gemm_kernel", grouped_gemm_kernel<C>, dim3(static_cast<unsigned>(grid)),
-                    dim3(C::THREADS), C::SMEM_BYTES, st, C::PAIR ? 2 : 1, a.R, map_a, map_b, p);
+                    dim3(C::THREADS), C::SMEM_BYTES, st, C::PAIR ? 2 : 1, a.R, map_a, map_a_small, map_b,
+                    p);
 }
 
 // ---- CUDA-core evaluation of the same contract (checking aid) --------------------------

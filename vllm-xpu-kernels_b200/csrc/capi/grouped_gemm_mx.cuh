@@ -56,8 +56,6 @@ struct MxConfig {
   static constexpr int A_BYTES = BM * kStageRowBytes;
   static constexpr int B_BYTES = BN * kStageRowBytes;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  // the barrier counts what TMA read: the packed 4-bit source, half of what lands in shared memory
-  static constexpr int STAGE_TX_BYTES = A_BYTES + B_BYTES / 2;
   static constexpr int B_ATOMS = (BN + 127) / 128;           // pieces copied per stage
   static constexpr int SFB_BYTES = B_ATOMS * kMxAtomBytes;
   static constexpr int COL_GROUPS = BN / 64;                 // reader warps per lane quadrant
@@ -150,6 +148,7 @@ __device__ __forceinline__ void mx_tile_epilogue(const MxParams& p, const TileCo
 template <typename C>
 __global__ void __launch_bounds__(C::THREADS, 1)
 grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
+                       const __grid_constant__ CUtensorMap map_a_small,
                        const __grid_constant__ CUtensorMap map_b,
                        const __grid_constant__ CUtensorMap map_b_tail, MxParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -182,6 +181,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
     }
     mbar_fence_init();
     prefetch_tensormap(&map_a);
+    prefetch_tensormap(&map_a_small);
     prefetch_tensormap(&map_b);
     prefetch_tensormap(&map_b_tail);
   }
@@ -208,6 +208,10 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
       for (int t = sched_id; t < num_tiles && ok; t += sched_stride) {
         const TileCoord tc = decode_tile(sched, t);
         const int n0 = tc.n_tile * C::BN;
+        const int small = small_boxes(tc.rows_valid);
+        // the barrier counts what TMA read: the packed 4-bit source, half of what lands in shared memory
+        const uint32_t stage_tx = (small ? small * (kSmallBox * kStageRowBytes) : C::A_BYTES) +
+                                  C::B_BYTES / 2 + C::SFB_BYTES;
         const uint8_t* sfb_tile =
             p.b_sf + (static_cast<int64_t>(tc.expert) * num_kb * p.b_atoms + n0 / 128) * kMxAtomBytes;
         for (int kb = 0; kb < num_kb && ok; ++kb) {
@@ -216,8 +220,13 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
           const bool tail = tail_skip && kb == num_kb - 1;
           uint8_t* a_dst = tiles + stage * C::STAGE_BYTES;
           if (elect_one()) {
-            mbar_arrive_expect_tx(&bars.full[stage], C::STAGE_TX_BYTES + C::SFB_BYTES);
-            tma_load_2d(a_dst, &map_a, &bars.full[stage], tail ? p.K - kMxBK : kb * kMxBK, tc.row_start);
+            mbar_arrive_expect_tx(&bars.full[stage], stage_tx);
+            const int ak = tail ? p.K - kMxBK : kb * kMxBK;
+            if (!small) tma_load_2d(a_dst, &map_a, &bars.full[stage], ak, tc.row_start);
+            else
+              for (int i = 0; i < small; ++i)
+                tma_load_2d(a_dst + i * (kSmallBox * kStageRowBytes), &map_a_small, &bars.full[stage], ak,
+                            tc.row_start + i * kSmallBox);
             if (tail) tma_load_3d(a_dst + C::A_BYTES, &map_b_tail, &bars.full[stage], 0, n0, tc.expert);
             else tma_load_3d(a_dst + C::A_BYTES, &map_b, &bars.full[stage], kb * kMxBK, n0, tc.expert);
             bulk_load(sfb_smem + stage * C::SFB_BYTES,
@@ -439,8 +448,9 @@ inline int make_map_fp4(CUtensorMap* map, const void* base, uint64_t cols, uint6
 
 template <typename C>
 int launch_mx(const b200moe_mx_gemm_args& a, cudaStream_t st) {
-  CUtensorMap map_a, map_b, map_b_tail;
+  CUtensorMap map_a, map_a_small, map_b, map_b_tail;
   int rc = make_map(&map_a, B200MOE_E4M3, a.A, a.K, a.R, 0, kMxBK, BM);
+  if (rc == B200MOE_OK) rc = make_map(&map_a_small, B200MOE_E4M3, a.A, a.K, a.R, 0, kMxBK, kSmallBox);
   if (rc != B200MOE_OK) return rc;
   const uint64_t pitch = static_cast<uint64_t>(a.K) / 2;
   const uint64_t k_main = static_cast<uint64_t>(a.K / kMxBK) * kMxBK;
@@ -477,7 +487,8 @@ int launch_mx(const b200moe_mx_gemm_args& a, cudaStream_t st) {
   if (grid > kNumSMs) grid = kNumSMs;
   if (grid < 1) grid = 1;
   return launch_pdl("grouped_gemm_mx_kernel", grouped_gemm_mx_kernel<C>, dim3(static_cast<unsigned>(grid)),
-                    dim3(C::THREADS), C::SMEM_BYTES, st, 1, a.R, map_a, map_b, map_b_tail, p);
+                    dim3(C::THREADS), C::SMEM_BYTES, st, 1, a.R, map_a, map_a_small,
+                    map_b, map_b_tail, p);
 }
 
 // Weight scales [E, N, K/32] (e8m0 bytes) -> [E, ceil(K/128), ceil(N/128)+1, 512]: per
