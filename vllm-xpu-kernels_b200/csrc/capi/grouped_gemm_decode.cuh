@@ -203,6 +203,7 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_tok,
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
+    const uint64_t policy = l2_evict_first();
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
       const DecodeTile tc = decode_tile(sched, t);
       for (int kb = 0; kb < num_kb && ok; ++kb) {
@@ -212,10 +213,10 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_tok,
         uint8_t* tok_dst = w_dst + C::W_TILES * kWBytes;
         if (elect_one()) {
           mbar_arrive_expect_tx(&bars.full[stage], C::STAGE_BYTES);
-          tma_load_3d(w_dst, &map_w, &bars.full[stage], tc.f_tile * kFeat, kb * kBK, tc.expert);
+          tma_load_3d_hint(w_dst, &map_w, &bars.full[stage], tc.f_tile * kFeat, kb * kBK, tc.expert, policy);
           if (GATED)
-            tma_load_3d(w_dst + kWBytes, &map_w, &bars.full[stage], p.N / 2 + tc.f_tile * kFeat,
-                        kb * kBK, tc.expert);
+            tma_load_3d_hint(w_dst + kWBytes, &map_w, &bars.full[stage], p.N / 2 + tc.f_tile * kFeat,
+                             kb * kBK, tc.expert, policy);
           tma_load_2d(tok_dst, &map_tok, &bars.full[stage], kb * kBK, tc.row_start);
         }
         __syncwarp();
