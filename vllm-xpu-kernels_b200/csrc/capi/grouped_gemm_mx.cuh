@@ -17,16 +17,23 @@
 // of MMAs into one accumulator buffer, and the reader warps only run epilogues
 // (bias, SwigluOAI, MXFP8 quantisation of the result for the second GEMM).
 //
-// Roles (one persistent CTA per SM): warp 0 TMA producer (A, B and SFB), warp 1 MMA
-// issuer, warp 2 activation-scale loader (the tile's 128 rows start at an arbitrary
-// row, so their scale words are fetched with plain loads, transposed into the
-// tensor-memory order in shared memory and published with a proxy fence), warps 4..
-// accumulator readers.  K need not be a multiple of 128: the last stage is loaded at
+// Roles (one persistent CTA per SM): warp 0 TMA producer (A and B), warp 1 MMA issuer,
+// warp 2 scale loader, warps 4.. accumulator readers.  Scales travel in groups of four
+// K blocks through a ring of their own: the tile's 128 rows start at an arbitrary row, so
+// their scale words are fetched with plain loads, transposed into the tensor-memory
+// order in shared memory and published with one proxy fence per group; the weight
+// scales of the group are two bulk copies.  (On the operand ring they cost the loader a fence
+// and two barrier waits, and the producer a third load, per K block.)  What bounds it: with many
+// rows the tensor pipe (384 cycles of MMAs per K block) and the issue loop that feeds it; with
+// few, the same loop at the clock that streaming from HBM leaves (128 experts, one row each,
+// N = 5760: 272 -> 248 us, 4.55 TB/s).  K need not be a multiple of 128: the last stage is loaded at
 // K-128 and only its new 32-wide sub-blocks are issued.
 
 constexpr int kMxBK = 128;            // elements of K per stage (128 bytes per row for both operands)
 constexpr int kMxSfaBytes = 512;      // one scale word per row of the A tile
 constexpr int kMxAtomBytes = 512;     // scales of 128 rows of B for one stage
+constexpr int kMxGroup = 4;           // K blocks per scale group
+constexpr int kMxSfGroups = 2;        // scale groups in flight
 constexpr int kMxSfaCol = 448;        // tensor-memory columns of the scale words
 constexpr int kMxSfbCol = 456;
 
@@ -34,7 +41,7 @@ struct MxParams {
   const uint8_t* a_sf;
   int64_t a_sf_pitch;
   const uint8_t* b_sf;  // prepared layout
-  int b_atoms;          // 128-row pieces per (expert, K block) in b_sf
+  int b_atoms;          // 128-row pieces per expert in b_sf
   const void* bias;
   int bias_dtype;
   void* D;
@@ -57,14 +64,14 @@ struct MxConfig {
   static constexpr int B_BYTES = BN * kStageRowBytes;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int B_ATOMS = (BN + 127) / 128;           // pieces copied per stage
-  static constexpr int SFB_BYTES = B_ATOMS * kMxAtomBytes;
+  static constexpr int SF_GROUP_BYTES = kMxGroup * (kMxSfaBytes + B_ATOMS * kMxAtomBytes);
   static constexpr int COL_GROUPS = BN / 64;                 // reader warps per lane quadrant
   static constexpr int EPI_WARPS = 4 * COL_GROUPS;
   static constexpr int THREADS = 128 + EPI_WARPS * 32;
   static constexpr int ACC_STRIDE = 256;                     // tensor-memory columns between the two accumulators
   static constexpr int TMEM_COLS = 512;
   static constexpr size_t SMEM_BYTES =
-      1024 + static_cast<size_t>(STAGES) * (STAGE_BYTES + kMxSfaBytes + SFB_BYTES);
+      1024 + static_cast<size_t>(STAGES) * STAGE_BYTES + kMxSfGroups * SF_GROUP_BYTES;
   static_assert(BN % 64 == 0 && BN <= 192, "two accumulators and the scale words share 512 columns");
   static_assert(STAGE_BYTES % 1024 == 0, "swizzled tiles start on 1 KiB boundaries");
 };
@@ -74,6 +81,8 @@ struct alignas(8) MxBarriers {
   uint64_t empty[8];
   uint64_t tfull[2];
   uint64_t tempty[2];
+  uint64_t sffull[kMxSfGroups];
+  uint64_t sfempty[kMxSfGroups];
 };
 
 // e8m0 byte of the smallest power of two >= max(amax, eps) / 448, floored like
@@ -95,12 +104,7 @@ __device__ __forceinline__ void mx_tile_epilogue(const MxParams& p, const TileCo
                                                  bool row_ok, int64_t grow, float (&acc)[64]) {
   const int col0 = tc.n_tile * C::BN + g * 64;  // first accumulator column of this thread
   if (col0 >= p.N) return;
-  if (p.bias) {
-#pragma unroll
-    for (int j = 0; j < 64; ++j)
-      if (col0 + j < p.N)
-        acc[j] += load_bias(p.bias, p.bias_dtype, static_cast<int64_t>(tc.expert) * p.N + col0 + j);
-  }
+  if (p.bias) add_bias_run<64>(p.bias, p.bias_dtype, static_cast<int64_t>(tc.expert) * p.N + col0, p.N - col0, acc);
   if constexpr (C::EPI == B200MOE_EPI_STORE) {
     if (row_ok) store_row16<64>(p.D, p.d_dtype, grow * p.ldd + col0, acc, p.N - col0);
   } else {  // SWIGLU_OAI: (gate, up) pairs are adjacent columns -> 32 results
@@ -159,8 +163,8 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
 
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
-  uint8_t* sfa_smem = tiles + C::STAGES * C::STAGE_BYTES;
-  uint8_t* sfb_smem = sfa_smem + C::STAGES * kMxSfaBytes;
+  // per scale group: four K blocks of row scales, then four of each piece of weight scales
+  uint8_t* sf_smem = tiles + C::STAGES * C::STAGE_BYTES;
   const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int n_tiles = (p.N + C::BN - 1) / C::BN;
@@ -172,8 +176,12 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
   if (threadIdx.x == 0) {
     abort_flag = 0;
     for (int s = 0; s < C::STAGES; ++s) {
-      mbar_init(&bars.full[s], 2);  // producer (with the byte count) + scale loader
+      mbar_init(&bars.full[s], 1);
       mbar_init(&bars.empty[s], 1);
+    }
+    for (int g = 0; g < kMxSfGroups; ++g) {
+      mbar_init(&bars.sffull[g], 1);
+      mbar_init(&bars.sfempty[g], 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&bars.tfull[b], 1);
@@ -200,139 +208,120 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
   const int sched_id = blockIdx.x, sched_stride = gridDim.x;
 
   if (warp == 0) {
-    {
-      // ---------------- TMA producer (warp-uniform loop, one elected lane issues) ----------------
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int t = sched_id; t < num_tiles && ok; t += sched_stride) {
-        const TileCoord tc = decode_tile(sched, t);
-        const int n0 = tc.n_tile * C::BN;
-        const int small = small_boxes(tc.rows_valid);
-        // the barrier counts what TMA read: the packed 4-bit source, half of what lands in shared memory
-        const uint32_t stage_tx = (small ? small * (kSmallBox * kStageRowBytes) : C::A_BYTES) +
-                                  C::B_BYTES / 2 + C::SFB_BYTES;
-        const uint8_t* sfb_tile =
-            p.b_sf + (static_cast<int64_t>(tc.expert) * num_kb * p.b_atoms + n0 / 128) * kMxAtomBytes;
-        for (int kb = 0; kb < num_kb && ok; ++kb) {
-          ok = mbar_wait_warp(&bars.empty[stage], phase ^ 1u, abort_p);
-          if (!ok) break;
-          const bool tail = tail_skip && kb == num_kb - 1;
-          uint8_t* a_dst = tiles + stage * C::STAGE_BYTES;
-          if (elect_one()) {
-            mbar_arrive_expect_tx(&bars.full[stage], stage_tx);
-            const int ak = tail ? p.K - kMxBK : kb * kMxBK;
-            if (!small) tma_load_2d(a_dst, &map_a, &bars.full[stage], ak, tc.row_start);
-            else
-              for (int i = 0; i < small; ++i)
-                tma_load_2d(a_dst + i * (kSmallBox * kStageRowBytes), &map_a_small, &bars.full[stage], ak,
-                            tc.row_start + i * kSmallBox);
-            if (tail) tma_load_3d(a_dst + C::A_BYTES, &map_b_tail, &bars.full[stage], 0, n0, tc.expert);
-            else tma_load_3d(a_dst + C::A_BYTES, &map_b, &bars.full[stage], kb * kMxBK, n0, tc.expert);
-            bulk_load(sfb_smem + stage * C::SFB_BYTES,
-                      sfb_tile + static_cast<int64_t>(kb) * p.b_atoms * kMxAtomBytes, C::SFB_BYTES,
-                      &bars.full[stage]);
-          }
-          __syncwarp();
-          if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
-        }
-      }
-    }
-  } else if (warp == 1) {
-    {
-      // ---------------- MMA issuer ----------------
-      // One thread feeds the tensor pipe, and an MMA of this shape takes about 100 cycles:
-      // the scalar instructions between two tcgen05.mma decide whether the pipe stays busy.
-      // So the stage index is a compile-time constant (the K loop is unrolled over the ring
-      // and runs across tile boundaries), every descriptor is a register base plus an
-      // immediate, and the instruction descriptors are constants.  Control flow around the
-      // MMAs is kept to whole blocks of straight-line issues: a per-instruction guard inside
-      // the unrolled loop (skip sub-block kk when kk < n) made the tail stage read the wrong
-      // sub-blocks whenever it fell on the first or last slot of the ring.
-      const uint32_t a0 = smem_u32(tiles);
-      const uint32_t sw_hi = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO 1024, version, 128-byte swizzle
-      const uint32_t sf_hi = (128u >> 4) | (1u << 14);                // SBO 128, version, no swizzle
-      const uint32_t a_lo0 = ((a0 & 0x3FFFFu) >> 4) | ((16u >> 4) << 16);
-      const uint32_t b_lo0 = a_lo0 + (C::A_BYTES >> 4);
-      const uint32_t sfa_lo0 = (smem_u32(sfa_smem) & 0x3FFFFu) >> 4;
-      const uint32_t sfb_lo0 = (smem_u32(sfb_smem) & 0x3FFFFu) >> 4;
-      const uint32_t sfa_t = tmem_base + kMxSfaCol;
-      auto desc = [](uint32_t lo, uint32_t hi) { return (static_cast<uint64_t>(hi) << 32) | lo; };
-      uint32_t phase = 0;
-      int buf = 0;
-      uint32_t buf_phase = 0;
-      bool ok = true;
-      int t = sched_id;
-      int kb = 0;
-      uint32_t d_tmem = 0, sfb_t = 0, accum = 0;
-      bool more = t < num_tiles;
-      while (more && ok) {
-#pragma unroll
-        for (int s = 0; s < C::STAGES; ++s) {
-          if (kb == 0) {
-            // next tile: its accumulator buffer must have been read out
-            const int n_tile = decode_tile(sched, t).n_tile;
-            // a tile that starts inside a 128-row piece of the scales (192-column tiles: every
-            // odd one starts at row 64) reads its scale columns from that offset on
-            sfb_t = tmem_base + kMxSfbCol + ((n_tile * C::BN) % 128) / 32;
-            ok = mbar_wait_warp(&bars.tempty[buf], buf_phase ^ 1u, abort_p);
-            if (!ok) break;
-            d_tmem = tmem_base + buf * C::ACC_STRIDE;
-            accum = 0;
-          }
-          ok = mbar_wait_warp(&bars.full[s], phase, abort_p);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t a_lo = a_lo0 + s * (C::STAGE_BYTES >> 4);
-          const uint32_t b_lo = b_lo0 + s * (C::STAGE_BYTES >> 4);
-          const bool last = kb == num_kb - 1;
-          if (elect_one()) {
-            tmem_cp_32x128b_x4(sfa_t, desc(sfa_lo0 + s * (kMxSfaBytes >> 4), sf_hi));
-#pragma unroll
-            for (int a = 0; a < C::B_ATOMS; ++a)
-              tmem_cp_32x128b_x4(tmem_base + kMxSfbCol + 4 * a,
-                                 desc(sfb_lo0 + (s * C::SFB_BYTES + a * kMxAtomBytes) / 16, sf_hi));
-            if (tail_skip && last) {
-              // K % 128 == 64 (rows of packed 4-bit weights have a 32-byte pitch, so K is a
-              // multiple of 64): the stage was loaded at K-128 and its first two sub-blocks were
-              // issued with the stage before
-              mma_mxf8f6f4(d_tmem, desc(a_lo + 4, sw_hi), desc(b_lo + 4, sw_hi),
-                           make_idesc_mx(0u, 5u, 0u, BM, C::BN, 2, 2), sfa_t, sfb_t, accum);
-              mma_mxf8f6f4(d_tmem, desc(a_lo + 6, sw_hi), desc(b_lo + 6, sw_hi),
-                           make_idesc_mx(0u, 5u, 0u, BM, C::BN, 3, 3), sfa_t, sfb_t, 1u);
-            } else {
-              mma_mxf8f6f4(d_tmem, desc(a_lo, sw_hi), desc(b_lo, sw_hi),
-                           make_idesc_mx(0u, 5u, 0u, BM, C::BN, 0, 0), sfa_t, sfb_t, accum);
-#pragma unroll
-              for (int kk = 1; kk < 4; ++kk)
-                mma_mxf8f6f4(d_tmem, desc(a_lo + kk * 2, sw_hi), desc(b_lo + kk * 2, sw_hi),
-                             make_idesc_mx(0u, 5u, 0u, BM, C::BN, kk, kk), sfa_t, sfb_t, 1u);
-            }
-            mma_commit(&bars.empty[s]);
-            if (last) mma_commit(&bars.tfull[buf]);
-          }
-          __syncwarp();
-          accum = 1;
-          if (++kb == num_kb) {
-            kb = 0;
-            if (++buf == 2) { buf = 0; buf_phase ^= 1u; }
-            t += sched_stride;
-            if (t >= num_tiles) { more = false; break; }
-          }
-        }
-        phase ^= 1u;
-      }
-    }
-  } else if (warp == 2) {
-    // ---------------- activation-scale loader ----------------
-    // Lane l owns rows l, 32+l, 64+l, 96+l of the tile.  One 16-byte load per row brings
-    // the scale words of four K blocks; they are fetched one group (four stages) ahead.
+    // ---------------- TMA producer (warp-uniform loop, one elected lane issues) ----------------
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
-    const int groups = (num_kb + 3) / 4;
-    auto load_group = [&](int t, int grp, uint4 (&w)[4]) {
+    for (int t = sched_id; t < num_tiles && ok; t += sched_stride) {
       const TileCoord tc = decode_tile(sched, t);
+      const int n0 = tc.n_tile * C::BN;
+      const int small = small_boxes(tc.rows_valid);
+      // the barrier counts what TMA read: the packed 4-bit source, half of what lands in shared memory
+      const uint32_t stage_tx = (small ? small * (kSmallBox * kStageRowBytes) : C::A_BYTES) + C::B_BYTES / 2;
+      for (int kb = 0; kb < num_kb && ok; ++kb) {
+        ok = mbar_wait_warp(&bars.empty[stage], phase ^ 1u, abort_p);
+        if (!ok) break;
+        const bool tail = tail_skip && kb == num_kb - 1;
+        uint8_t* a_dst = tiles + stage * C::STAGE_BYTES;
+        if (elect_one()) {
+          mbar_arrive_expect_tx(&bars.full[stage], stage_tx);
+          const int ak = tail ? p.K - kMxBK : kb * kMxBK;
+          if (!small) tma_load_2d(a_dst, &map_a, &bars.full[stage], ak, tc.row_start);
+          else
+            for (int i = 0; i < small; ++i)
+              tma_load_2d(a_dst + i * (kSmallBox * kStageRowBytes), &map_a_small, &bars.full[stage], ak,
+                          tc.row_start + i * kSmallBox);
+          if (tail) tma_load_3d(a_dst + C::A_BYTES, &map_b_tail, &bars.full[stage], 0, n0, tc.expert);
+          else tma_load_3d(a_dst + C::A_BYTES, &map_b, &bars.full[stage], kb * kMxBK, n0, tc.expert);
+        }
+        __syncwarp();
+        if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer ----------------
+    // The 384 cycles of MMAs per K block (the scale copies hide behind them) leave no room for a
+    // slow issue loop: a plain loop whose descriptors are base + stage * constant, on values the
+    // compiler knows to be warp-uniform.  (Unrolled over the ring, with the tensor-memory base
+    // as a per-lane value out of shared memory, issuing alone took 520 of 620 cycles.)
+    // Whole blocks of straight-line issues, chosen by a uniform branch, are kept: a
+    // per-instruction guard between MMAs once issued wrong sub-blocks.
+    const uint32_t a0 = smem_u32(tiles);
+    const uint32_t sw_hi = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO 1024, version, 128-byte swizzle
+    const uint32_t sf_hi = (128u >> 4) | (1u << 14);                // SBO 128, version, no swizzle
+    const uint32_t a_lo0 = ((a0 & 0x3FFFFu) >> 4) | ((16u >> 4) << 16);
+    const uint32_t sf_lo0 = (smem_u32(sf_smem) & 0x3FFFFu) >> 4;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+    const uint32_t sfa_t = tmem + kMxSfaCol;
+    auto desc = [](uint32_t lo, uint32_t hi) { return (static_cast<uint64_t>(hi) << 32) | lo; };
+    uint32_t stage = 0, phase = 0;
+    uint32_t buf = 0, buf_phase = 0;
+    uint32_t sg = 0, sg_phase = 0;   // scale group in use
+    bool ok = true;
+    for (int t = sched_id; t < num_tiles && ok; t += sched_stride) {
+      // a tile that starts inside a 128-row piece of the scales (192-column tiles: every odd one
+      // starts at row 64) reads its scale columns from that offset on
+      const int n_tile = __shfl_sync(0xffffffffu, decode_tile(sched, t).n_tile, 0);
+      const uint32_t sfb_t = tmem + kMxSfbCol + ((n_tile * C::BN) % 128) / 32;
+      ok = mbar_wait_warp(&bars.tempty[buf], buf_phase ^ 1u, abort_p);
+      if (!ok) break;
+      const uint32_t d_tmem = tmem + buf * C::ACC_STRIDE;
+      uint32_t accum = 0;
+      for (int kb = 0; kb < num_kb && ok; ++kb) {
+        const uint32_t j = static_cast<uint32_t>(kb) % kMxGroup;
+        const bool last = kb == num_kb - 1;
+        if (j == 0) {
+          ok = mbar_wait_warp(&bars.sffull[sg], sg_phase, abort_p);
+          if (!ok) break;
+        }
+        ok = mbar_wait_warp(&bars.full[stage], phase, abort_p);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t sf_lo = sf_lo0 + (sg * C::SF_GROUP_BYTES + j * kMxSfaBytes) / 16;
+        const uint32_t a_lo = a_lo0 + stage * (C::STAGE_BYTES >> 4);
+        const uint32_t b_lo = a_lo + (C::A_BYTES >> 4);
+        if (elect_one()) {
+          tmem_cp_32x128b_x4(sfa_t, desc(sf_lo, sf_hi));
+#pragma unroll
+          for (int a = 0; a < C::B_ATOMS; ++a)
+            tmem_cp_32x128b_x4(tmem + kMxSfbCol + 4 * a, desc(sf_lo + (1 + a) * (kMxGroup * kMxAtomBytes / 16), sf_hi));
+          if (tail_skip && last) {
+            // K % 128 == 64 (rows of packed 4-bit weights have a 32-byte pitch, so K is a
+            // multiple of 64): the stage was loaded at K-128 and its first two sub-blocks were
+            // issued with the stage before
+            mma_mxf8f6f4(d_tmem, desc(a_lo + 4, sw_hi), desc(b_lo + 4, sw_hi),
+                         make_idesc_mx(0u, 5u, 0u, BM, C::BN, 2, 2), sfa_t, sfb_t, accum);
+            mma_mxf8f6f4(d_tmem, desc(a_lo + 6, sw_hi), desc(b_lo + 6, sw_hi),
+                         make_idesc_mx(0u, 5u, 0u, BM, C::BN, 3, 3), sfa_t, sfb_t, 1u);
+          } else {
+            mma_mxf8f6f4(d_tmem, desc(a_lo, sw_hi), desc(b_lo, sw_hi),
+                         make_idesc_mx(0u, 5u, 0u, BM, C::BN, 0, 0), sfa_t, sfb_t, accum);
+#pragma unroll
+            for (int kk = 1; kk < 4; ++kk)
+              mma_mxf8f6f4(d_tmem, desc(a_lo + kk * 2, sw_hi), desc(b_lo + kk * 2, sw_hi),
+                           make_idesc_mx(0u, 5u, 0u, BM, C::BN, kk, kk), sfa_t, sfb_t, 1u);
+          }
+          mma_commit(&bars.empty[stage]);
+          if (last) mma_commit(&bars.tfull[buf]);
+          if (last || j == kMxGroup - 1) mma_commit(&bars.sfempty[sg]);   // the group has been copied
+        }
+        __syncwarp();
+        accum = 1;
+        if (last || j == kMxGroup - 1) {
+          if (++sg == kMxSfGroups) { sg = 0; sg_phase ^= 1u; }
+        }
+        if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
+      }
+      if (++buf == 2) { buf = 0; buf_phase ^= 1u; }
+    }
+  } else if (warp == 2) {
+    // ---------------- scale loader ----------------
+    // Lane l owns rows l, 32+l, 64+l, 96+l of the tile.  One 16-byte load per row brings
+    // the scale words of a group; they are fetched one group ahead.
+    uint32_t sg = 0, sg_phase = 1;
+    bool ok = true;
+    const int groups = (num_kb + kMxGroup - 1) / kMxGroup;
+    auto load_group = [&](const TileCoord& tc, int grp, uint4 (&w)[4]) {
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         int64_t row = static_cast<int64_t>(tc.row_start) + c * 32 + lane;
@@ -344,23 +333,33 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
     uint4 cur[4], nxt[4];
     uint32_t prev_last[4] = {0u, 0u, 0u, 0u};
     int t = sched_id;
-    if (t < num_tiles) load_group(t, 0, nxt);
+    TileCoord tc{}, tc_next{};
+    if (t < num_tiles) {
+      tc_next = decode_tile(sched, t);
+      load_group(tc_next, 0, nxt);
+    }
     for (; t < num_tiles && ok; t += sched_stride) {
+      tc = tc_next;
+      if (t + sched_stride < num_tiles) tc_next = decode_tile(sched, t + sched_stride);
+      const uint8_t* sfb = p.b_sf + (static_cast<int64_t>(tc.expert) * p.b_atoms + tc.n_tile * C::BN / 128) *
+                                        num_kb * kMxAtomBytes;
       for (int grp = 0; grp < groups && ok; ++grp) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) cur[c] = nxt[c];
-        if (grp + 1 < groups) load_group(t, grp + 1, nxt);
-        else if (t + sched_stride < num_tiles) load_group(t + sched_stride, 0, nxt);
+        if (grp + 1 < groups) load_group(tc, grp + 1, nxt);
+        else if (t + sched_stride < num_tiles) load_group(tc_next, 0, nxt);
+        ok = mbar_wait_warp(&bars.sfempty[sg], sg_phase, abort_p);
+        if (!ok) break;
+        uint8_t* dst = sf_smem + sg * C::SF_GROUP_BYTES;
+        const int n = num_kb - grp * kMxGroup < kMxGroup ? num_kb - grp * kMxGroup : kMxGroup;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int kb = grp * 4 + j;
-          if (kb >= num_kb) break;
+        for (int j = 0; j < kMxGroup; ++j) {
           uint4 o;
           uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             uint32_t v = word(cur[c], j);
-            if (tail_skip && kb == num_kb - 1) {
+            if (tail_skip && grp * kMxGroup + j == num_kb - 1) {
               // bytes of sub-blocks [K/32 - 4, K/32): the last (4 - tail_skip) bytes of the
               // previous word followed by the first tail_skip... of this one
               const uint32_t before = j > 0 ? word(cur[c], j - 1) : prev_last[c];
@@ -368,16 +367,22 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a,
             }
             ow[c] = v;
           }
-          ok = mbar_wait_spin(&bars.empty[stage], phase ^ 1u, abort_p);
-          if (!ok) break;
-          *reinterpret_cast<uint4*>(sfa_smem + stage * kMxSfaBytes + lane * 16) = o;
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars.full[stage]);
-          if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
+          if (j < n) *reinterpret_cast<uint4*>(dst + j * kMxSfaBytes + lane * 16) = o;
         }
 #pragma unroll
         for (int c = 0; c < 4; ++c) prev_last[c] = cur[c].w;
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (elect_one()) {
+          mbar_arrive_expect_tx(&bars.sffull[sg], C::B_ATOMS * n * kMxAtomBytes);
+#pragma unroll
+          for (int a = 0; a < C::B_ATOMS; ++a)
+            bulk_load(dst + (1 + a) * (kMxGroup * kMxAtomBytes),
+                      sfb + (static_cast<int64_t>(a) * num_kb + grp * kMxGroup) * kMxAtomBytes, n * kMxAtomBytes,
+                      &bars.sffull[sg]);
+        }
+        __syncwarp();
+        if (++sg == kMxSfGroups) { sg = 0; sg_phase ^= 1u; }
       }
     }
   } else if (warp >= 4) {
@@ -491,8 +496,8 @@ int launch_mx(const b200moe_mx_gemm_args& a, cudaStream_t st) {
                     map_b, map_b_tail, p);
 }
 
-// Weight scales [E, N, K/32] (e8m0 bytes) -> [E, ceil(K/128), ceil(N/128)+1, 512]: per
-// (expert, K block, 128 rows) the 512 bytes tcgen05.cp wants, byte (n%32)*16 + (n%128/32)*4 + j
+// Weight scales [E, N, K/32] (e8m0 bytes) -> [E, ceil(N/128)+1, ceil(K/128), 512]: per
+// (expert, 128 rows, K block) the 512 bytes tcgen05.cp wants, byte (n%32)*16 + (n%128/32)*4 + j
 // holding the scale of row n and sub-block j of that K block.  A last K block that starts at
 // K-128 gets the sub-blocks it really covers.  Rows past N and the extra piece hold 1.0.
 __global__ void mx_prepare_weight_scales_kernel(const uint8_t* __restrict__ s, uint8_t* __restrict__ out,
@@ -504,10 +509,10 @@ __global__ void mx_prepare_weight_scales_kernel(const uint8_t* __restrict__ s, u
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int in_atom = static_cast<int>(i % 128);  // word index: lane * 4 + column
     int64_t rest = i / 128;
-    const int atom = static_cast<int>(rest % atoms);
-    rest /= atoms;
     const int kb = static_cast<int>(rest % num_kb);
-    const int e = static_cast<int>(rest / num_kb);
+    rest /= num_kb;
+    const int atom = static_cast<int>(rest % atoms);
+    const int e = static_cast<int>(rest / atoms);
     const int n = atom * 128 + (in_atom & 3) * 32 + (in_atom >> 2);
     const int sub0 = (kb == num_kb - 1 && (K % kMxBK)) ? sub_total - 4 : kb * 4;
     uint32_t w = 0;
