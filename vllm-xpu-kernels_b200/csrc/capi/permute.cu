@@ -217,9 +217,11 @@ __global__ void __launch_bounds__(kThreads) fused_small_kernel(GroupParams p, Al
 // The same for any number of indices: one cluster of kGroupCtas CTAs.  Bound by latency, not
 // by bytes (0.5 MB of indices at 16384 tokens x 8): what counts is the number of dependent
 // steps.  Three launches (count, scan over per-CTA counts, place) took 16 us at 18 k indices
-// and 26 us at 131 k; here the counts never leave shared memory.
+// and 26 us at 131 k; here the counts never leave shared memory.  The walks take the time (a warp
+// match per 32 indices), so as many warps as a cluster holds share them: 1024 threads a CTA
+// against 512 measured 59 -> 44 us at 131 k indices, 14.7 -> 10.7 at 33 k.
 constexpr int kGroupCtas = 8;
-constexpr int kGroupThreads = 512;
+constexpr int kGroupThreads = 1024;
 constexpr int kGroupWarps = kGroupThreads / 32;
 
 __global__ void __cluster_dims__(kGroupCtas, 1, 1) __launch_bounds__(kGroupThreads)
@@ -258,7 +260,8 @@ group_cluster_kernel(GroupParams p, AlignOut ao, int32_t* __restrict__ rows_per_
     if (key >= 0) atomicAdd(&mine[key], 1);
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < K; e += kGroupThreads) {
+  if (threadIdx.x < K) {
+    const int e = threadIdx.x;
     int run = 0;
     for (int w = 0; w < kGroupWarps; ++w) {
       const int c = smem[w * K + e];
@@ -268,30 +271,21 @@ group_cluster_kernel(GroupParams p, AlignOut ao, int32_t* __restrict__ rows_per_
     total[e] = run;
   }
   cluster.sync();
-  int before[2] = {0, 0};   // of keys threadIdx.x and threadIdx.x + 512: counts of the CTAs before this one
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const int e = threadIdx.x + j * kGroupThreads;
-    if (e >= K) break;
-    int sum = 0;
+  static_assert(kGroupThreads >= kMaxExperts, "one thread per key");
+  const int e = threadIdx.x;   // this thread's key
+  int before = 0, grand = 0;   // its count in the CTAs before this one, and in all
+  if (e < K) {
 #pragma unroll
     for (int c = 0; c < kGroupCtas; ++c) {
       const int v = cluster.map_shared_rank(total, c)[e];
-      if (c < rank) before[j] += v;
-      sum += v;
+      if (c < rank) before += v;
+      grand += v;
     }
-    grand_of[e] = sum;
+    grand_of[e] = grand;
   }
-  __syncthreads();
-  // exclusive scan of the padded counts over the keys, two neighbouring keys per thread
+  // exclusive scan of the padded counts over the keys
   {
-    int v[2], local = 0;
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int e = threadIdx.x * 2 + j;
-      v[j] = e < K ? (grand_of[e] + p.block_size - 1) / p.block_size * p.block_size : 0;
-      local += v[j];
-    }
+    const int local = (grand + p.block_size - 1) / p.block_size * p.block_size;
     int incl = local;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
@@ -302,18 +296,12 @@ group_cluster_kernel(GroupParams p, AlignOut ao, int32_t* __restrict__ rows_per_
     __syncthreads();
     int base = 0;
     for (int w = 0; w < warp; ++w) base += warp_sums[w];
-    const int e0 = threadIdx.x * 2;
-    if (e0 < K) start[e0] = base + incl - local;
-    if (e0 + 1 < K) start[e0 + 1] = base + incl - v[1];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const int e = threadIdx.x + j * kGroupThreads;
-    if (e >= K) break;
-    const int add = start[e] + before[j];
-    for (int w = 0; w < kGroupWarps; ++w) smem[w * K + e] += add;
-    if (rank == 0 && rows_per_key) rows_per_key[e] = (accumulate ? rows_per_key[e] : 0) + grand_of[e];
+    if (e < K) {
+      start[e] = base + incl - local;
+      const int add = base + incl - local + before;
+      for (int w = 0; w < kGroupWarps; ++w) smem[w * K + e] += add;
+      if (rank == 0 && rows_per_key) rows_per_key[e] = (accumulate ? rows_per_key[e] : 0) + grand;
+    }
   }
   __syncthreads();
   auto place = [&](int key, int64_t idx) {
@@ -344,13 +332,13 @@ group_cluster_kernel(GroupParams p, AlignOut ao, int32_t* __restrict__ rows_per_
     const int last = K - 1;
     const int all = start[last] + (grand_of[last] + p.block_size - 1) / p.block_size * p.block_size;
     const int32_t pad = static_cast<int32_t>(p.numel);
-    for (int e = rank * kGroupWarps + warp; e < K; e += kGroupCtas * kGroupWarps) {
-      const int n = grand_of[e];
-      const int end = start[e] + (n + p.block_size - 1) / p.block_size * p.block_size;
-      for (int i = start[e] + n + lane; i < end; i += 32)
+    for (int x = rank * kGroupWarps + warp; x < K; x += kGroupCtas * kGroupWarps) {
+      const int n = grand_of[x];
+      const int end = start[x] + (n + p.block_size - 1) / p.block_size * p.block_size;
+      for (int i = start[x] + n + lane; i < end; i += 32)
         if (i < ao.sorted_capacity) ao.sorted_ids[i] = pad;
-      const int label = ao.expert_map ? ao.expert_map[e] : e;
-      for (int b = start[e] / p.block_size + lane; b < end / p.block_size; b += 32)
+      const int label = ao.expert_map ? ao.expert_map[x] : x;
+      for (int b = start[x] / p.block_size + lane; b < end / p.block_size; b += 32)
         if (b < ao.blocks_capacity) ao.expert_ids[b] = label;
     }
     const int64_t gid = rank * kGroupThreads + threadIdx.x;
