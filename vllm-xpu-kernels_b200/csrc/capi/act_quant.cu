@@ -209,33 +209,35 @@ __device__ __forceinline__ void fetch8(const T* __restrict__ in, int64_t r, int 
 
 // FP8 e4m3 group quantisation.  DIVIDE selects q = x / s (fused SiLU op)
 // versus q = x * (1/s) (stand-alone op).  Streaming; what bounded it was not HBM but the work per
-// chunk (64-bit divisions for the row and column, a runtime-length shuffle, one 16-byte load in
-// flight): 16384 x 7168 bf16 took 188 us, 1.9 TB/s.  LANES is the group in threads of 8
-// elements (0: run-time), UNROLL chunks are in flight per thread, and contiguous scales need no
-// row number at all.
-template <typename T, bool SILU, bool DIVIDE, int LANES>
+// element (64-bit divisions for the row and column, a runtime-length shuffle, one 16-byte load in
+// flight): 16384 x 7168 bf16 took 188 us, 1.9 TB/s; with eight elements a thread and four
+// threads' worth in flight 114, with sixteen and 16-byte stores 78.  LANES is the group in
+// threads of PER elements (0: run-time); contiguous scales need no row number at all.
+template <typename T, bool SILU, bool DIVIDE, int LANES, int PER>
 __global__ void __launch_bounds__(256) group_quant_fp8_kernel(
     const T* __restrict__ in, uint8_t* __restrict__ out_q, float* __restrict__ out_s, uint32_t total,
     int64_t first_row, uint32_t chunks_per_row, int lanes_rt, float eps, float fp8_min, float fp8_max, bool ue8m0,
     const float* __restrict__ scale_ub, int64_t ss_row, int64_t ss_group) {
-  constexpr int UNROLL = SILU ? 2 : 4;
+  constexpr int UNROLL = 2, H = PER / kVec;
   const int lanes = LANES ? LANES : lanes_rt;
-  const int N = static_cast<int>(chunks_per_row) * kVec;
+  const int N = static_cast<int>(chunks_per_row) * PER;
   const float min_scale = 1.0f / (fp8_max * 512.0f);
   const int64_t in_base = first_row * N * (SILU ? 2 : 1);
   pdl_wait();
   pdl_trigger();
-  float x[UNROLL][kVec];
+  float x[UNROLL][H][kVec];
   const uint32_t base = blockIdx.x * (256u * UNROLL) + threadIdx.x;
 #pragma unroll
   for (int u = 0; u < UNROLL; ++u) {
     const uint32_t c = base + u * 256u;
     if (c < total) {
-      if constexpr (SILU) {
-        const uint32_t r = c / chunks_per_row;
-        fetch8<T, true>(in + in_base, r, static_cast<int>(c - r * chunks_per_row) * kVec, N, x[u]);
-      } else {
-        fetch8<T, false>(in + in_base + static_cast<int64_t>(c) * kVec, 0, 0, N, x[u]);
+      const uint32_t r = SILU ? c / chunks_per_row : 0u;
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        if constexpr (SILU)
+          fetch8<T, true>(in + in_base, r, static_cast<int>(c - r * chunks_per_row) * PER + h * kVec, N, x[u][h]);
+        else
+          fetch8<T, false>(in + in_base + static_cast<int64_t>(c) * PER + h * kVec, 0, 0, N, x[u][h]);
       }
     }
   }
@@ -246,7 +248,7 @@ __global__ void __launch_bounds__(256) group_quant_fp8_kernel(
     float amax = 0.f;
     if (live) {
 #pragma unroll
-      for (int i = 0; i < kVec; ++i) amax = fmaxf(amax, fabsf(x[u][i]));
+      for (int i = 0; i < PER; ++i) amax = fmaxf(amax, fabsf(x[u][i / kVec][i % kVec]));
     }
     amax = LANES ? seg_max<LANES ? LANES : 1>(amax) : seg_max_dyn(amax, lanes);
     float s = SILU ? amax / fp8_max : fmaxf(amax, eps) / fp8_max;
@@ -255,25 +257,31 @@ __global__ void __launch_bounds__(256) group_quant_fp8_kernel(
     if (ue8m0) s = round_up_pow2(s);
     if (!live) continue;
     if ((threadIdx.x & 31) % lanes == 0) {
-      const uint32_t group = c / static_cast<uint32_t>(lanes), per_row = chunks_per_row / lanes;
-      const uint32_t r = group / per_row;
-      out_s[(first_row + r) * ss_row + static_cast<int64_t>(group - r * per_row) * ss_group] = s;
+      const uint32_t group = c / static_cast<uint32_t>(lanes);
+      if (ss_group == 1 && ss_row == static_cast<int64_t>(chunks_per_row / lanes)) {
+        out_s[first_row * ss_row + group] = s;
+      } else {
+        const uint32_t per_row = chunks_per_row / lanes, r = group / per_row;
+        out_s[(first_row + r) * ss_row + static_cast<int64_t>(group - r * per_row) * ss_group] = s;
+      }
     }
     const float inv = 1.0f / s;
-    uint32_t q[2];
+    uint32_t q[PER / 4];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < PER / 4; ++h) {
       float y[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float v = x[u][4 * h + i];
+        const float v = x[u][(4 * h) / kVec][(4 * h) % kVec + i];
         y[i] = fmaxf(fp8_min, fminf(DIVIDE ? v / s : v * inv, fp8_max));
       }
       const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(y[0], y[1]), __NV_SATFINITE, __NV_E4M3);
       const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(y[2], y[3]), __NV_SATFINITE, __NV_E4M3);
       q[h] = lo | (hi << 16);
     }
-    *reinterpret_cast<uint2*>(out_q + first_row * N + static_cast<int64_t>(c) * kVec) = make_uint2(q[0], q[1]);
+    uint8_t* dst = out_q + first_row * N + static_cast<int64_t>(c) * PER;
+    if constexpr (PER == 16) *reinterpret_cast<uint4*>(dst) = make_uint4(q[0], q[1], q[2], q[3]);
+    else *reinterpret_cast<uint2*>(dst) = make_uint2(q[0], q[1]);
   }
 }
 
@@ -439,20 +447,24 @@ template <typename T, bool SILU, bool DIVIDE>
 static int launch_group_quant(const void* in, void* out_q, float* out_s, int64_t R, int N, int group_size, float eps,
                               float fp8_min, float fp8_max, bool ue8m0, const float* scale_ub, int64_t ss_row,
                               int64_t ss_group, void* stream) {
-  constexpr unsigned kPerBlock = 256u * (SILU ? 2 : 4);
-  const int64_t chunks = N / kVec, most = ((1ll << 31) - 1) / chunks;
+  // 16 elements a thread where a group is whole threads of 16 and the codes can leave in 16-byte
+  // stores
+  const bool wide = group_size % 16 == 0 && reinterpret_cast<uintptr_t>(out_q) % 16 == 0;
+  const int per = wide ? 16 : kVec;
+  const int64_t chunks = N / per, most = ((1ll << 31) - 1) / chunks;
   for (int64_t r0 = 0; r0 < R; r0 += most) {
     const int64_t rows = R - r0 < most ? R - r0 : most;
     const uint32_t total = static_cast<uint32_t>(rows * chunks);
     auto go = [&](auto kernel) {
-      return launch_pdl("group_quant_fp8_kernel", kernel, dim3((total + kPerBlock - 1) / kPerBlock), dim3(256), 0,
+      return launch_pdl("group_quant_fp8_kernel", kernel, dim3((total + 511) / 512), dim3(256), 0,
                         as_stream(stream), 1, rows, reinterpret_cast<const T*>(in), reinterpret_cast<uint8_t*>(out_q),
-                        out_s, total, r0, static_cast<uint32_t>(chunks), group_size / kVec, eps, fp8_min, fp8_max,
+                        out_s, total, r0, static_cast<uint32_t>(chunks), group_size / per, eps, fp8_min, fp8_max,
                         ue8m0, scale_ub, ss_row, ss_group);
     };
-    const int rc = group_size == 128 ? go(group_quant_fp8_kernel<T, SILU, DIVIDE, 16>)
-                   : group_size == 32 ? go(group_quant_fp8_kernel<T, SILU, DIVIDE, 4>)
-                                      : go(group_quant_fp8_kernel<T, SILU, DIVIDE, 0>);
+    const int rc = wide && group_size == 128 ? go(group_quant_fp8_kernel<T, SILU, DIVIDE, 8, 16>)
+                   : wide && group_size == 32 ? go(group_quant_fp8_kernel<T, SILU, DIVIDE, 2, 16>)
+                   : wide                     ? go(group_quant_fp8_kernel<T, SILU, DIVIDE, 0, 16>)
+                                              : go(group_quant_fp8_kernel<T, SILU, DIVIDE, 0, 8>);
     if (rc != B200MOE_OK) return rc;
   }
   return B200MOE_OK;
