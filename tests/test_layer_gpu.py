@@ -232,6 +232,24 @@ def test_few_tokens_take_the_decode_kernels(ops, T, monkeypatch):
     check(out2, ref, 2e-2)
 
 
+@pytest.mark.parametrize("T", [5, 32, 33])
+def test_enough_weights_and_at_most_32_tokens_take_the_decode_kernels(ops, T, monkeypatch):
+    """8 experts of 37 feature tiles are just enough for the second half of the rule; 33 tokens are
+    one too many.  All tokens choose the same two experts, so that a chunk is full at 32."""
+    monkeypatch.delenv("B200MOE_DECODE_PATH", raising=False)
+    cfg = dict(O.CONFIGS["c1"], H=256, I=37 * 128)
+    layer = O.make_layer(cfg, T=T)
+    layer["logits"][:, 2:4] += 100.0
+    moe = build(cfg, layer)
+    w, ids = route_gpu(ops, cfg, layer)
+    rw, rids = O.route(cfg, layer)
+    out = torch.empty(T, cfg["H"], dtype=torch.bfloat16, device=DEV)
+    moe.apply(out, to_dev(layer["x"]), w, ids)
+    ref = O.fused_moe("fp8block", layer["x"], layer["w13"], layer["w13_scale"], None, layer["w2"],
+                      layer["w2_scale"], None, rw, rids, "silu", out_dtype=torch.float32)
+    check(out, ref, 2e-2)
+
+
 @pytest.mark.parametrize("T", [3, 200])
 def test_shared_expert_added_in_the_combine(ops, T):
     """A DeepSeek-V3-style layer: routed experts plus one shared expert every token passes

@@ -529,11 +529,10 @@ class XpuFusedMoe:
         return gemm2_out
 
     def _decode_regime(self, routed_rows: int) -> bool:
-        """Whether to run the two GEMMs on the decode-regime kernel (weights on the M side of
-        the MMA, 32 tokens per tile).  With at most about one routed row per local expert it is
-        4-6 % faster end to end on the DeepSeek-V3 shape (1..32 tokens); from a few rows per
-        expert on, hot experts need several 32-token chunks that each stream the weights again,
-        and the 128-row-tile kernel wins.  B200MOE_DECODE_PATH=0/1 overrides."""
+        """Whether ``apply`` runs the two GEMMs on the decode-regime kernel (weights on the M side
+        of the MMA, 32 tokens per tile): with at most about one routed row per local expert, or,
+        on a layer with enough weights, with at most 32 tokens, which is decided in native code
+        (`decode_regime` in layer.cu gives the figures).  B200MOE_DECODE_PATH=0/1 overrides."""
         forced = os.environ.get("B200MOE_DECODE_PATH")
         if forced is not None:
             return forced == "1"
