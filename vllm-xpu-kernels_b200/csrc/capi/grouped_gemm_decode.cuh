@@ -136,7 +136,10 @@ template <bool GATED>
 struct DecodeConfig {
   static constexpr int W_TILES = GATED ? 2 : 1;
   static constexpr int STAGE_BYTES = W_TILES * kWBytes + kTokBytes;
-  static constexpr int STAGES = GATED ? 5 : 8;
+  // 128 or 96 KB of weights in flight per SM.  More only queue: with 5 and 8 stages one token on the
+  // DeepSeek-V3 shape took 92.1 us, with 4 and 6 88.7 (64 tokens 1711 -> 1637), with 4 and 5 the
+  // same, with 2 and 4 95.3.
+  static constexpr int STAGES = GATED ? 4 : 6;
   static constexpr int ACC_COLS = 64;   // per buffer: gate 32 | up 32 (plain uses the first 32)
   static constexpr int ACC_BUFS = 4;
   static constexpr int TMEM_COLS = 256;
