@@ -232,9 +232,9 @@ def test_few_tokens_take_the_decode_kernels(ops, T, monkeypatch):
     check(out2, ref, 2e-2)
 
 
-@pytest.mark.parametrize("T", [5, 32, 33])
-def test_enough_weights_and_at_most_32_tokens_take_the_decode_kernels(ops, T, monkeypatch):
-    """8 experts of 37 feature tiles are just enough for the second half of the rule; 33 tokens are
+@pytest.mark.parametrize("T", [5, 32, 33, 64, 65])
+def test_enough_weights_and_few_tokens_take_the_decode_kernels(ops, T, monkeypatch):
+    """8 experts of 37 feature tiles are just enough for the second half of the rule; 65 tokens are
     one too many.  All tokens choose the same two experts, so that a chunk is full at 32."""
     monkeypatch.delenv("B200MOE_DECODE_PATH", raising=False)
     cfg = dict(O.CONFIGS["c1"], H=256, I=37 * 128)

@@ -45,21 +45,24 @@ Workspace carve(const b200moe_layer* l, const b200moe_layer_call* c) {
 // When the block-FP8 GEMMs run on the decode-regime kernel (weights on the M side of the MMA, 32
 // tokens per tile).  Two conditions, either is enough:
 //  - about one routed row per local expert: 4-6 % faster end to end on the DeepSeek-V3 shape;
-//  - at most 32 tokens, so that no expert, however skewed the routing, has more than one 32-token
-//    chunk and no weight is streamed twice.  The 128-row-tile kernel multiplies 128 rows for those
-//    few and runs into the power limit over it: Mixtral, 16 tokens 301 -> 264 us, 32 tokens
-//    309 -> 268, DeepSeek-V3, 16 tokens 964 -> 827, 32 tokens 1525 -> 1294.  With more tokens hot
-//    experts decide (DeepSeek-V3, 128 skewed tokens 499 -> 551), and the host does not see them.
+//  - at most 64 tokens, so that no expert, however skewed the routing, has more than two 32-token
+//    chunks, which run next to each other and read the weights from L2 the second time.  The
+//    128-row-tile kernel multiplies 128 rows for those few and runs into the power limit over it:
+//    Mixtral, 16 tokens 301 -> 264 us, 64 tokens 312 -> 279, 64 skewed tokens 282 -> 274;
+//    DeepSeek-V3, 16 tokens 946 -> 790, 64 tokens 2124 -> 1729, 64 skewed tokens 450 -> 419.  With
+//    more tokens hot experts decide (96 skewed tokens on Mixtral 318 -> 355, on DeepSeek-V3
+//    483 -> 487), and the host does not see them.
 //    Not for layers whose tiles of 128 features do not fill the SMs twice over (8 experts of 2048:
 //    30.3 -> 32.8 us at 64 tokens) and not for power-of-two scales, which the other kernel applies
-//    in the tensor core (Mixtral, 16 tokens: medians 269 and 262 us, best runs 245 and 250).
+//    in the tensor core (Mixtral, 64 tokens 257 us against 266 here, 64 skewed tokens 226 against
+//    263).
 bool decode_regime(const b200moe_layer* l, const b200moe_layer_call* c) {
   if (l->recipe != B200MOE_RECIPE_FP8_BLOCK || l->gated_act != B200MOE_ACT_SILU || l->clamp_limit > 0.0f ||
       c->valid_tokens)
     return false;
   if (const char* forced = getenv("B200MOE_DECODE_PATH")) return forced[0] == '1' && forced[1] == 0;
   if (static_cast<int64_t>(c->T) * c->k <= l->E) return true;
-  return c->T <= 32 && !l->scales_pow2 && static_cast<int64_t>(l->E) * (l->I / 128) >= 2 * kNumSMs;
+  return c->T <= 64 && !l->scales_pow2 && static_cast<int64_t>(l->E) * (l->I / 128) >= 2 * kNumSMs;
 }
 
 int gemm(const b200moe_layer* l, const b200moe_layer_call* c, const Workspace& w, uint8_t* ws, bool second,

@@ -531,7 +531,7 @@ class XpuFusedMoe:
     def _decode_regime(self, routed_rows: int) -> bool:
         """Whether ``apply`` runs the two GEMMs on the decode-regime kernel (weights on the M side
         of the MMA, 32 tokens per tile): with at most about one routed row per local expert, or,
-        on a layer with enough weights, with at most 32 tokens, which is decided in native code
+        on a layer with enough weights, with at most 64 tokens, which is decided in native code
         (`decode_regime` in layer.cu gives the figures).  B200MOE_DECODE_PATH=0/1 overrides."""
         forced = os.environ.get("B200MOE_DECODE_PATH")
         if forced is not None:
