@@ -59,6 +59,20 @@ def test_per_token_group_fp8_quant(ops, R, N, gs, dtype, ue8m0):
     assert torch.equal(st.cpu(), rs)
 
 
+@pytest.mark.parametrize("R,N,gs,shift", [(1, 16, 16, 0), (33, 512, 256, 0), (7, 48, 8, 0), (65, 1152, 128, 8)])
+def test_fp8_group_quant_thread_widths(ops, R, N, gs, shift):
+    """Sixteen elements a thread where a group and the output address allow it, eight elsewhere."""
+    x = torch.randn(R, N, generator=torch.Generator().manual_seed(gs)).to(torch.bfloat16)
+    rq, rs = O.per_token_group_fp8_quant(x, gs, 1e-10, False)
+    q = torch.zeros(R * N + 16, dtype=torch.uint8, device=DEV)
+    s = torch.empty(R, N // gs, dtype=torch.float32, device=DEV)
+    ops._C.per_token_group_fp8_quant(x.to(DEV), q[shift:shift + R * N].view(torch.float8_e4m3fn).view(R, N), s, gs,
+                                     1e-10, -448.0, 448.0, False, False, False)
+    assert torch.equal(s.cpu(), rs)
+    assert torch.equal(q[shift:shift + R * N].cpu().view(R, N), rq.view(torch.uint8))
+    assert (q[:shift] == 0).all() and (q[shift + R * N:] == 0).all()
+
+
 def test_fp8_group_quant_golden(ops):
     g = load_golden("fp8_group")
     q = torch.empty(16, 512, dtype=torch.float8_e4m3fn, device=DEV)

@@ -78,6 +78,21 @@ def test_rows_beyond_an_expert_are_untouched(ops):
     close(D[:135], ref)
 
 
+@pytest.mark.parametrize("rows_list", [[1, 32, 33], [64, 65, 96], [97, 127, 128], [129, 160, 225]])
+def test_tiles_with_few_rows(ops, rows_list):
+    """A tile of at most 96 rows loads its activations in boxes of 32 rows; the rest of the operand
+    buffer keeps what it held."""
+    E, K, N = len(rows_list), 320, 256
+    rows = torch.tensor(rows_list, dtype=torch.int32)
+    R = int(rows.sum())
+    A = torch.randn(R, K, generator=torch.Generator().manual_seed(R)).to(torch.bfloat16)
+    B = make_bf16(E, K, N, 4)
+    D = torch.full((R + 2, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops._xpu_C.b200_grouped_gemm(A.to(DEV), None, B.to(DEV), None, None, D, rows.to(DEV), N, K, E, EPI_STORE, KN)
+    close(D[:R], O.grouped_gemm("bf16", A, B, None, None, rows, torch.float32))
+    assert (D[R:] == 7.0).all()
+
+
 @pytest.mark.parametrize("epi", [EPI_SILU, EPI_OAI])
 @pytest.mark.parametrize("layout", [KN, NK])
 @pytest.mark.parametrize("E,avg,K,N", [(4, 90, 256, 512), (8, 40, 1024, 4096), (2, 150, 192, 5760)])

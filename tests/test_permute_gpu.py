@@ -64,6 +64,16 @@ def test_align_with_a_permuted_expert_map(ops, T, k, E, bs):
     assert torch.equal(t, rt) and torch.equal(e, re) and torch.equal(s, rs)
 
 
+@pytest.mark.parametrize("numel,E", [(2047, 1), (2048, 1024), (2049, 1024), (8193, 257), (65535, 3), (262145, 31)])
+def test_align_where_the_walks_of_the_cluster_end(ops, numel, E):
+    """One CTA up to 2048 indices, a cluster above; its warps walk equal runs of the indices, the
+    last of them short or empty, and one thread serves one expert (1024 at most)."""
+    ids = torch.randint(0, E, (numel, 1), generator=torch.Generator().manual_seed(numel)).to(torch.int32)
+    rs, re, rt = O.moe_align_block_size(ids, 16, E)
+    s, e, t = run_align(ops, ids, 16, E)
+    assert torch.equal(t, rt) and torch.equal(e, re) and torch.equal(s, rs)
+
+
 def test_align_skewed_and_out_of_range(ops):
     ids = torch.zeros(5000, 4, dtype=torch.int32)       # every token on expert 0
     ids[::7, 1] = 99                                     # ids >= num_experts are ignored
@@ -143,6 +153,21 @@ def test_gather_and_sum_vs_oracle(ops, T, k, H, dtype):
         out = torch.empty(T, H, dtype=dtype, device=DEV)
         ops._moe_C.moe_sum(x3.to(DEV), out, *[None if a is None else a.to(DEV) for a in args])
         assert torch.allclose(out.cpu().float(), ref.float(), atol=2e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("T,k,H", [(1, 1, 8), (3, 3, 8200), (129, 9, 264), (600, 17, 520)])
+def test_combine_in_batches_of_source_rows(ops, T, k, H):
+    """k without an instantiation of its own goes through in batches of eight, the last one short;
+    columns are numbered across row boundaries."""
+    g = torch.Generator().manual_seed(k)
+    y = torch.randn(T * k, H, generator=g).to(torch.bfloat16)
+    w = torch.rand(T, k, generator=g)
+    rmap = torch.randperm(T * k, generator=g).view(T, k).to(torch.int32)
+    out = torch.empty(T, H, dtype=torch.bfloat16, device=DEV)
+    ops._moe_C.moe_gather(out, y.to(DEV), w.to(DEV), rmap.to(DEV), 8)
+    assert torch.allclose(out.cpu().float(), O.moe_gather(y, w, rmap).float(), atol=2e-2, rtol=2e-2)
+    ops._moe_C.moe_sum(y.view(T, k, H).to(DEV), out, None, None)
+    assert torch.allclose(out.cpu().float(), O.moe_sum(y.view(T, k, H)).float(), atol=3e-2, rtol=2e-2)
 
 
 def test_moe_sum_input_validation(ops):
