@@ -155,16 +155,20 @@ def test_gather_and_sum_vs_oracle(ops, T, k, H, dtype):
         assert torch.allclose(out.cpu().float(), ref.float(), atol=2e-2, rtol=2e-2)
 
 
-@pytest.mark.parametrize("T,k,H", [(1, 1, 8), (3, 3, 8200), (129, 9, 264), (600, 17, 520)])
-def test_combine_in_batches_of_source_rows(ops, T, k, H):
+@pytest.mark.parametrize("T,k,H,shift", [(1, 1, 8, 0), (3, 3, 8200, 0), (129, 9, 264, 0), (600, 17, 520, 0),
+                                         (295, 8, 6144, 0), (296, 8, 6144, 0), (297, 8, 6144, 1), (40, 4, 1024, 1)])
+def test_combine_in_batches_of_source_rows(ops, T, k, H, shift):
     """k without an instantiation of its own goes through in batches of eight, the last one short;
-    columns are numbered across row boundaries."""
+    columns are numbered across row boundaries; eight rows of many tokens take two columns a thread
+    (from 296 tokens of 6144); row numbers and weights need not start on 16 bytes."""
     g = torch.Generator().manual_seed(k)
     y = torch.randn(T * k, H, generator=g).to(torch.bfloat16)
     w = torch.rand(T, k, generator=g)
     rmap = torch.randperm(T * k, generator=g).view(T, k).to(torch.int32)
+    rmap[torch.rand(T, k, generator=g) < 0.2] = -1
     out = torch.empty(T, H, dtype=torch.bfloat16, device=DEV)
-    ops._moe_C.moe_gather(out, y.to(DEV), w.to(DEV), rmap.to(DEV), 8)
+    dw, dm = (torch.empty(T * k + shift, dtype=a.dtype, device=DEV)[shift:].view(T, k).copy_(a) for a in (w, rmap))
+    ops._moe_C.moe_gather(out, y.to(DEV), dw, dm, 8)
     assert torch.allclose(out.cpu().float(), O.moe_gather(y, w, rmap).float(), atol=2e-2, rtol=2e-2)
     ops._moe_C.moe_sum(y.view(T, k, H).to(DEV), out, None, None)
     assert torch.allclose(out.cpu().float(), O.moe_sum(y.view(T, k, H)).float(), atol=3e-2, rtol=2e-2)

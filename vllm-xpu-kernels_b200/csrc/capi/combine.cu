@@ -24,34 +24,55 @@ struct CombineParams {
   int ids_dtype;
   const int32_t* expert_map;  // sum, optional
   int k, H, vecs;             // vecs: columns of V elements per row
+  bool aligned;               // gather: row_map and weights start on 16 bytes
   int64_t t0;                 // first token of this launch
   uint32_t total;             // (token, column) pairs of this launch
 };
 
-// K: rows per token when known at compile time (0: k, in batches of kAhead).
-template <typename T, int V, int K, bool GATHER>
-__global__ void __launch_bounds__(256) combine_kernel(CombineParams p) {
+// K: rows per token when known at compile time (0: k, in batches of kAhead).  C: columns per
+// thread.  A thread's time is two round trips, the row numbers and then the rows, so with many
+// tokens what counts is how many threads come one after the other and what the row numbers cost:
+// with eight rows two columns share them, read as two 16-byte loads each.  16384 tokens of
+// 8 x 7168: 464 -> 430 us (4.9 TB/s); 4099 tokens with one row in eight present: 69 -> 56.  Two
+// columns of four or six rows measured slower (43 -> 52 us, 17 -> 19), as did registers for a third
+// CTA per SM (430 -> 729).
+template <typename T, int V, int K, bool GATHER, int C>
+__global__ void __launch_bounds__(256, C == 2 ? 2 : 1) combine_kernel(CombineParams p) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   pdl_wait();
   pdl_trigger();
   if (i >= p.total) return;
-  const uint32_t local = i / static_cast<uint32_t>(p.vecs);
+  const uint32_t per_row = static_cast<uint32_t>(p.vecs) / C;
+  const uint32_t local = i / per_row;
   const int64_t t = p.t0 + local;
   if (GATHER && p.num_valid && t >= *p.num_valid) return;  // rows of a worst-case buffer nobody will read
-  const int64_t c = static_cast<int64_t>(i - local * p.vecs) * V;
+  const int64_t c = static_cast<int64_t>(i - local * per_row) * V;
+  const int64_t next = static_cast<int64_t>(per_row) * V;  // from a thread's column to its next
   const int k = K ? K : p.k;
   const T* in = reinterpret_cast<const T*>(p.in);
-  float acc[V];
-  if (GATHER && p.addend) {  // e.g. the shared expert's row of this token, weight 1
-    load_f32<T, V>(reinterpret_cast<const T*>(p.addend) + t * p.H + c, acc);
-  } else {
+  float acc[C][V];
 #pragma unroll
-    for (int e = 0; e < V; ++e) acc[e] = 0.f;
+  for (int q = 0; q < C; ++q) {
+    if (GATHER && p.addend) {  // e.g. the shared expert's row of this token, weight 1
+      load_f32<T, V>(reinterpret_cast<const T*>(p.addend) + t * p.H + c + q * next, acc[q]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < V; ++e) acc[q][e] = 0.f;
+    }
   }
   constexpr int B = K ? K : kAhead;
   for (int j0 = 0; j0 < k; j0 += B) {
-    int64_t row[B];
+    int32_t row[B];
     float w[B];
+    if (GATHER && K % 4 == 0 && K && p.aligned) {
+#pragma unroll
+      for (int j = 0; j < B; j += 4) {
+        const int4 r4 = *reinterpret_cast<const int4*>(p.row_map + t * k + j);
+        const float4 w4 = *reinterpret_cast<const float4*>(p.weights + t * k + j);
+        row[j] = r4.x; row[(j + 1) % B] = r4.y; row[(j + 2) % B] = r4.z; row[(j + 3) % B] = r4.w;
+        w[j] = w4.x; w[(j + 1) % B] = w4.y; w[(j + 2) % B] = w4.z; w[(j + 3) % B] = w4.w;
+      }
+    } else {
 #pragma unroll
     for (int j = 0; j < B; ++j) {
       row[j] = -1;
@@ -62,7 +83,7 @@ __global__ void __launch_bounds__(256) combine_kernel(CombineParams p) {
           row[j] = p.row_map[at];
           w[j] = p.weights[at];
         } else {
-          row[j] = at;
+          row[j] = j0 + j;
           if (p.ids) {
             const int64_t id = load_index(p.ids, p.ids_dtype, at);
             if (id < 0 || (p.expert_map && p.expert_map[id] < 0)) row[j] = -1;
@@ -70,43 +91,55 @@ __global__ void __launch_bounds__(256) combine_kernel(CombineParams p) {
         }
       }
     }
-    Vec<T, V> v[B];
-#pragma unroll
-    for (int j = 0; j < B; ++j)
-      if (row[j] >= 0) v[j] = *reinterpret_cast<const Vec<T, V>*>(in + row[j] * p.H + c);
+    }
+    const T* base = GATHER ? in + c : in + t * k * p.H + c;
+    Vec<T, V> v[B][C];
 #pragma unroll
     for (int j = 0; j < B; ++j)
       if (row[j] >= 0) {
 #pragma unroll
-        for (int e = 0; e < V; ++e) {
-          const float x = Elem<T>::to_f32(v[j].v[e]);
-          acc[e] += GATHER ? w[j] * x : x;
-        }
+        for (int q = 0; q < C; ++q)
+          v[j][q] = *reinterpret_cast<const Vec<T, V>*>(base + static_cast<int64_t>(row[j]) * p.H + q * next);
+      }
+#pragma unroll
+    for (int j = 0; j < B; ++j)
+      if (row[j] >= 0) {
+#pragma unroll
+        for (int q = 0; q < C; ++q)
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            const float x = Elem<T>::to_f32(v[j][q].v[e]);
+            acc[q][e] += GATHER ? w[j] * x : x;
+          }
       }
   }
-  store_f32<T, V>(reinterpret_cast<T*>(p.out) + t * p.H + c, acc);
+#pragma unroll
+  for (int q = 0; q < C; ++q) store_f32<T, V>(reinterpret_cast<T*>(p.out) + t * p.H + c + q * next, acc[q]);
 }
 
 template <typename T, int V, bool GATHER>
 int launch_combine(CombineParams p, int T_, cudaStream_t st) {
   p.vecs = p.H / V;
+  p.aligned = ((reinterpret_cast<uintptr_t>(p.row_map) | reinterpret_cast<uintptr_t>(p.weights)) & 15) == 0;
   const int64_t most = ((1ll << 31) - 1) / p.vecs;   // tokens per launch: pair numbers stay below 2^31
   for (int64_t t0 = 0; t0 < T_; t0 += most) {
     const int64_t n = T_ - t0 < most ? T_ - t0 : most;
     p.t0 = t0;
-    p.total = static_cast<uint32_t>(n * p.vecs);
+    // two columns a thread where that still leaves every SM three CTAs' worth of them
+    const bool two = p.k == 8 && p.vecs % 2 == 0 && n * p.vecs >= 2ll * 3 * 256 * kNumSMs;
+    p.total = static_cast<uint32_t>(n * p.vecs / (two ? 2 : 1));
     // few tokens: smaller CTAs, so that more SMs pull
     const int threads = p.total < 256u * kNumSMs ? 64 : 256;
     const dim3 grid((p.total + threads - 1) / threads);
     auto go = [&](auto kernel) { return launch_pdl("combine_kernel", kernel, grid, dim3(threads), 0, st, 1, n * p.k, p); };
     int rc;
     switch (p.k) {
-      case 1: rc = go(combine_kernel<T, V, 1, GATHER>); break;
-      case 2: rc = go(combine_kernel<T, V, 2, GATHER>); break;
-      case 4: rc = go(combine_kernel<T, V, 4, GATHER>); break;
-      case 6: rc = go(combine_kernel<T, V, 6, GATHER>); break;
-      case 8: rc = go(combine_kernel<T, V, 8, GATHER>); break;
-      default: rc = go(combine_kernel<T, V, 0, GATHER>); break;
+      case 1: rc = go(combine_kernel<T, V, 1, GATHER, 1>); break;
+      case 2: rc = go(combine_kernel<T, V, 2, GATHER, 1>); break;
+      case 4: rc = go(combine_kernel<T, V, 4, GATHER, 1>); break;
+      case 6: rc = go(combine_kernel<T, V, 6, GATHER, 1>); break;
+      case 8: rc = two ? go(combine_kernel<T, V, 8, GATHER, 2>) : go(combine_kernel<T, V, 8, GATHER, 1>); break;
+      default: rc = go(combine_kernel<T, V, 0, GATHER, 1>); break;
     }
     if (rc != B200MOE_OK) return rc;
   }
